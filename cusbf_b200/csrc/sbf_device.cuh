@@ -56,14 +56,13 @@ __device__ __forceinline__ uint64_t salt(int j) {
 // earliest byte first: byte r lands at bits (31-2r):(30-2r).
 __device__ __forceinline__ uint32_t pack4_top(uint32_t c) { return c * 0x40100401u; }
 
-__device__ __forceinline__ uint32_t invalid4(uint32_t v, uint32_t c) {
-    // Expected upper-case letter for each byte's code: table A C T G indexed
-    // by the code; a byte is valid exactly when (byte & 0xDF) equals it.
-    const uint32_t s = c | (c >> 4);
-    const uint32_t e_lo = __byte_perm(0x47544341u, 0u, s);
-    const uint32_t e_hi = __byte_perm(0x47544341u, 0u, s >> 16);
-    const uint32_t expect = __byte_perm(e_lo, e_hi, 0x5410u);
-    return (v & 0xDFDFDFDFu) ^ expect;  // non-zero byte <=> invalid base
+// Non-zero in the bits of kInvalidMask of every byte of `v` that is not a base.
+// Without bits 1 and 2 (the code) and 5 (the case) a base reads 0x41, or 0x50
+// when its code is 2 (T): three instructions on the logic pipe for four bytes.
+constexpr uint32_t kInvalidMask = 0xD9D9D9D9u;
+__device__ __forceinline__ uint32_t invalid4(uint32_t v) {
+    const uint32_t is_t = (v >> 2) & ~(v >> 1) & 0x01010101u;
+    return v ^ (is_t * 0x11u) ^ 0x41414141u;
 }
 
 __device__ __forceinline__ uint32_t nonzero_bytes_to_bits(uint32_t d) {
@@ -80,15 +79,17 @@ __device__ __forceinline__ void encode16(uint32_t v0, uint32_t v1, uint32_t v2, 
     const uint32_t lo = __byte_perm(pack4_top(c3), pack4_top(c2), 0x0073u);
     const uint32_t hi = __byte_perm(pack4_top(c1), pack4_top(c0), 0x0073u);
     code = __byte_perm(lo, hi, 0x5410u);
-    const uint32_t d0 = invalid4(v0, c0);
-    const uint32_t d1 = invalid4(v1, c1);
-    const uint32_t d2 = invalid4(v2, c2);
-    const uint32_t d3 = invalid4(v3, c3);
-    if ((d0 | d1 | d2 | d3) == 0u) {
+    const uint32_t d0 = invalid4(v0);
+    const uint32_t d1 = invalid4(v1);
+    const uint32_t d2 = invalid4(v2);
+    const uint32_t d3 = invalid4(v3);
+    if (((d0 | d1 | d2 | d3) & kInvalidMask) == 0u) {
         inval = 0u;
     } else {
-        inval = nonzero_bytes_to_bits(d0) | (nonzero_bytes_to_bits(d1) << 4) |
-                (nonzero_bytes_to_bits(d2) << 8) | (nonzero_bytes_to_bits(d3) << 12);
+        inval = nonzero_bytes_to_bits(d0 & kInvalidMask) |
+                (nonzero_bytes_to_bits(d1 & kInvalidMask) << 4) |
+                (nonzero_bytes_to_bits(d2 & kInvalidMask) << 8) |
+                (nonzero_bytes_to_bits(d3 & kInvalidMask) << 12);
     }
 }
 

@@ -16,11 +16,27 @@ constexpr int kTileKmers = kThreads * kStrip;          // k-mers per tile (8192)
 constexpr int kStripWords = kStrip / 16 + 2;           // code words one strip reads
 constexpr int kCodeWords = (kThreads - 1) * (kStrip / 16) + kStripWords;  // per tile
 constexpr int kStageBytes = kCodeWords * 16 + 64;      // staged input bytes per buffer
-constexpr int kSlots = 10;                             // query shard slots per thread
-constexpr int kOverflow = 6;                           // deferred shard loads per thread
-constexpr int kQuerySlotBytes = kSlots * kThreads * 32 + kOverflow * kThreads * 4;
 constexpr int kFlushSlots = 8;                         // insert bulk-reduce staging slots
 constexpr int kInsertSlotBytes = kFlushSlots * kThreads * 32;  // dynamic smem of inserts
+
+// A warp's dynamic shared memory in the query kernels: a pool of shard slots
+// (first the run lists of its lanes, 32 entries each) and the shard id of
+// every slot.  A warp of random sequence needs 121 slots at W = 16 m-mers a
+// window and 171 at W = 11 (the runs of 32 strips less the borrowed ones),
+// with a deviation of 6 to 8; a warp that needs more takes several rounds.
+// Three CTAs of 256 threads and 80 registers fit an SM with 208 slots a warp;
+// shorter windows change runs more often (252 slots at W = 8) and longer ones
+// and more than eight hashes need more registers, so those run two CTAs.
+// Run-time compilation takes device functions only.
+#ifdef __CUDACC_RTC__
+#define SBF_SIZE_FN __device__ constexpr
+#else
+#define SBF_SIZE_FN constexpr
+#endif
+SBF_SIZE_FN bool query_three_ctas(int w, int h) { return w >= 10 && w <= 16 && h <= 8; }
+SBF_SIZE_FN int query_pool_slots(int w, int h) { return query_three_ctas(w, h) ? 208 : 344; }
+SBF_SIZE_FN int query_warp_bytes(int w, int h) { return query_pool_slots(w, h) * (32 + 4); }
+SBF_SIZE_FN int query_cta_bytes(int w, int h) { return kThreads / 32 * query_warp_bytes(w, h); }
 
 // A record of a ragged launch: bytes [offset, offset + bytes) of the input.
 // Same layout as sbf_record_range of the C ABI.
@@ -103,9 +119,9 @@ struct KernelSet {
     const void* insert_ragged;
     const void* query_ragged;
     // Dynamic shared memory of the insert and query kernels: the tile
-    // kernels' flush ring and shard slots; none for the generic kernels.
+    // kernels' flush ring and shard pool; none for the generic kernels.
     int smem_insert = kInsertSlotBytes;
-    int smem_query = kQuerySlotBytes;
+    int smem_query = query_cta_bytes(k - m + 1, h);
     bool jit = false;    // loaded from a run-time compiled library
     int jit_occupancy = 2;  // resident CTAs per SM assumed for run-time compiled sets
     int smem(bool query) const { return query ? smem_query : smem_insert; }

@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(kThreads, 2) emit_kernel(TileParams p, RunLog 
         __syncthreads();
         for (int q = tid; q < kCodeWords; q += kThreads) {
             uint32_t cw, iv;
-            encode_word<false>(g, stage, q, cw, iv);
+            encode_word<false>(g.off, stage, q, cw, iv);
             code[q] = cw;
             inval[q] = iv;
         }
@@ -83,7 +83,10 @@ __global__ void __launch_bounds__(kThreads, 2) emit_kernel(TileParams p, RunLog 
             iv[q] = inval[tid * (kStrip / 16) + q];
         }
         const int64_t first_kmer = g.s0 + static_cast<int64_t>(tid) * kStrip;
-        const uint32_t vmask = strip_valid<C>(iv, first_kmer, p.n_kmers);
+        const uint64_t bits = static_cast<uint64_t>(iv[0]) | (static_cast<uint64_t>(iv[1]) << 16) |
+                              (static_cast<uint64_t>(iv[2]) << 32) |
+                              (static_cast<uint64_t>(iv[3]) << 48);
+        const uint32_t vmask = strip_valid<C>(bits, first_kmer, p.n_kmers);
         n_valid += __popc(vmask);
         if (vmask)
             insert_strip<C>(c, vmask, p.shard_mask, onehot, [&](uint32_t end, uint32_t shard,

@@ -8,10 +8,10 @@
 // and their dense-packed twins).  Results are bit-identical to it; the work
 // decomposition is new:
 //
-//   * A persistent CTA (two per SM) walks tiles of 8192 consecutive windows
+//   * A persistent CTA (two or three per SM) walks tiles of 8192 consecutive windows
 //     (kTileKmers).  Each tile's input bytes are staged into shared memory by
-//     a 1D bulk async copy (TMA) on an mbarrier, double-buffered and issued
-//     two tiles ahead, so copies overlap hashing.  Only the 16-byte aligned
+//     a 1D bulk async copy (TMA) on an mbarrier, issued as soon as the tile
+//     before it is encoded, so copies overlap hashing.  Only the 16-byte aligned
 //     interior goes through the bulk copy; ragged edges are read with plain
 //     loads, so nothing outside the caller's buffer is touched.  Every wait
 //     is bounded and reports kDevErrStageTimeout instead of hanging.
@@ -21,16 +21,17 @@
 //     m-mer and s-mer of the strip is a funnel shift of the code words,
 //     every position is hashed once, and the per-window minimizer is a
 //     Gil-Werman sliding minimum over blocks of W positions (about 3
-//     comparisons per window for any W <= 16, where the reference hashes
+//     comparisons per window, one more for W > 16, where the reference hashes
 //     and compares all W m-mers of every window).
 //   * Insert merges consecutive windows that select the same shard (a
 //     super-k-mer run) in registers and flushes each run with one 32-byte
 //     bulk OR-reduction (cp.reduce.async.bulk .or.b64) from a per-thread
 //     shared-memory ring: one L2 sector operation per run.
-//   * Query copies each run head's 32-byte shard into per-thread shared
-//     slots with cp.async as the heads are found, borrows the left
-//     neighbour's staged shard when a run crosses the strip boundary, and
-//     tests the findere rule (all k-s+1 s-mers present) per window.
+//   * Query lists each strip's runs, gives the runs that hold a valid window
+//     consecutive slots of a per-warp shared-memory pool, and has the warp
+//     copy their 32-byte shards there with cp.async, a lane pair per shard
+//     (one request each).  It then tests the findere rule (all k-s+1 s-mers
+//     present) per window with byte permutes of the current run's shard.
 //   * Insert word masks come from a shared one-hot table (1 << b).
 //   * Ragged launches take tiles from a device work-queue counter and drop
 //     windows that cross a record boundary or touch a byte outside every
@@ -71,10 +72,14 @@ struct TileGeom {
     int64_t s0;      // symbol index of the tile's first grid position
 };
 
+__device__ __forceinline__ int64_t tile_first_symbol(const TileParams& p, uint64_t tile) {
+    return static_cast<int64_t>(tile) * kTileKmers + p.sym_base;
+}
+
 template <bool kDense>
 __device__ __forceinline__ TileGeom tile_geom(const TileParams& p, uint64_t tile) {
     TileGeom g;
-    g.s0 = static_cast<int64_t>(tile) * kTileKmers + p.sym_base;
+    g.s0 = tile_first_symbol(p, tile);
     uint32_t need;
     if constexpr (kDense) {
         // 2-bit symbols: symbol s sits at bit 2s of the byte stream.
@@ -107,8 +112,10 @@ __device__ __forceinline__ TileGeom tile_geom(const TileParams& p, uint64_t tile
     return g;
 }
 
+// Starts the tile's staging copy; returns whether it covers the whole stage
+// window (every tile but those at the input's ends).
 template <bool kDense>
-__device__ __forceinline__ void issue_stage(const TileParams& p, uint64_t tile, uint8_t* buf,
+__device__ __forceinline__ bool issue_stage(const TileParams& p, uint64_t tile, uint8_t* buf,
                                             uint64_t* bar) {
     const TileGeom g = tile_geom<kDense>(p, tile);
     fence_proxy_async_smem();
@@ -119,6 +126,7 @@ __device__ __forceinline__ void issue_stage(const TileParams& p, uint64_t tile, 
     } else {
         mbar_arrive(bar);
     }
+    return g.lo == g.a && g.hi == g.a + g.span;
 }
 
 // Plain loads of the readable bytes of the stage window that the bulk copy
@@ -150,20 +158,28 @@ __device__ __forceinline__ void fill_ragged(const TileParams& p, const TileGeom&
     }
 }
 
+// Where grid position 0 lies in the stage: its byte, or its bit for dense
+// input.  The same for every tile, since a tile is a multiple of 16 bytes.
+template <bool kDense>
+__device__ __forceinline__ uint32_t stage_origin(const TileParams& p) {
+    const TileGeom g = tile_geom<kDense>(p, 0);
+    return kDense ? 8u * g.off + 2u * static_cast<uint32_t>(g.s0 - 4 * g.b_lo) : g.off;
+}
+static_assert(kTileKmers / 4 % 16 == 0, "tiles start at one phase of 16 bytes");
+
 // Encodes code word q (16 symbols from grid position 16q) of the staged tile.
 template <bool kDense>
-__device__ __forceinline__ void encode_word(const TileGeom& g, const uint8_t* buf, int q,
+__device__ __forceinline__ void encode_word(uint32_t origin, const uint8_t* buf, int q,
                                             uint32_t& code, uint32_t& inval) {
     const uint32_t* w32 = reinterpret_cast<const uint32_t*>(buf);
     if constexpr (kDense) {
-        const int64_t sym_in_stage = g.s0 - 4 * g.b_lo;  // 0..3
-        const uint32_t bitpos = 8u * g.off + 2u * static_cast<uint32_t>(sym_in_stage) + 32u * q;
+        const uint32_t bitpos = origin + 32u * q;
         const uint32_t wi = bitpos >> 5;
         const uint32_t v = __funnelshift_r(w32[wi], w32[wi + 1], bitpos & 31u);
         code = dense16_to_code(v);
         inval = 0u;
     } else {
-        const uint32_t bytepos = g.off + 16u * q;
+        const uint32_t bytepos = origin + 16u * q;
         const uint32_t wi = bytepos >> 2;
         const uint32_t sh = (bytepos & 3u) * 8u;
         const uint32_t x0 = w32[wi], x1 = w32[wi + 1], x2 = w32[wi + 2], x3 = w32[wi + 3],
@@ -211,69 +227,79 @@ __device__ __forceinline__ uint64_t smer_at(const uint32_t* c, int r) {
     }
 }
 
-// Low word of min(a, b): the shard only needs the minimum's low 32 bits.
-__device__ __forceinline__ uint32_t min64_lo(uint64_t a, uint64_t b) {
-    return static_cast<uint32_t>(a < b ? a : b);
-}
-
-// Calls fn(j, shard) for the strip's windows j = 0..kStrip-1 in order.
-// For 2 <= W <= 16 m-mers per window the minimum is a Gil-Werman sliding
-// minimum over blocks of W positions: window b0 + r of the block starting at
-// b0 is min(suffix_b0[r], prefix_{b0+W}[r-1]), about three 64-bit
-// comparisons per window whatever W is (instead of W - 1).
-template <class C, class Fn>
-__device__ __forceinline__ void for_each_shard(const uint32_t* c, uint32_t shard_mask, Fn&& fn) {
-    constexpr int W = C::W;
-    if constexpr (W >= 2 && W <= 16) {
+// Calls fn(j, v) for j = 0..N-1 in order, v being the minimum hash of the W
+// m-mers from position j on (2 <= W <= 16): a Gil-Werman sliding minimum over
+// blocks of W positions.  Window b0 + r of the block starting at b0 is
+// min(suffix_b0[r], prefix_{b0+W}[r-1]), about three 64-bit comparisons per
+// window whatever W is (instead of W - 1).
+template <class C, int W, int N, class Fn>
+__device__ __forceinline__ void sliding_min(const uint32_t* c, Fn&& fn) {
 #pragma unroll
-        for (int b0 = 0; b0 < kStrip; b0 += W) {
-            uint64_t suf[W];
-            suf[W - 1] = mh_at<C>(c, b0 + W - 1);
+    for (int b0 = 0; b0 < N; b0 += W) {
+        uint64_t suf[W];
+        suf[W - 1] = mh_at<C>(c, b0 + W - 1);
 #pragma unroll
-            for (int r = W - 2; r >= 0; --r) suf[r] = min64(mh_at<C>(c, b0 + r), suf[r + 1]);
-            fn(b0, static_cast<uint32_t>(suf[0]) & shard_mask);
-            uint64_t pre = ~uint64_t{0};
+        for (int r = W - 2; r >= 0; --r) suf[r] = min64(mh_at<C>(c, b0 + r), suf[r + 1]);
+        fn(b0, suf[0]);
+        uint64_t pre = ~uint64_t{0};
 #pragma unroll
-            for (int r = 1; r < W; ++r) {
-                if (b0 + r < kStrip) {
-                    pre = min64(pre, mh_at<C>(c, b0 + W - 1 + r));
-                    fn(b0 + r, min64_lo(suf[r], pre) & shard_mask);
-                }
+        for (int r = 1; r < W; ++r) {
+            if (b0 + r < N) {
+                pre = min64(pre, mh_at<C>(c, b0 + W - 1 + r));
+                fn(b0 + r, min64(suf[r], pre));
             }
         }
-    } else {
-#pragma unroll
-        for (int j = 0; j < kStrip; ++j) {
-            uint64_t v = mh_at<C>(c, j);
-#pragma unroll
-            for (int o = 1; o < W; ++o) v = min64(v, mh_at<C>(c, j + o));
-            fn(j, static_cast<uint32_t>(v) & shard_mask);
-        }
     }
+}
+
+// Calls fn(j, lo) for the strip's windows j = 0..kStrip-1 in order, lo being
+// the low word of the window's minimum m-mer hash (its shard id, unmasked).
+// Windows of more than 16 m-mers take the minimum of their first and their
+// last 16.
+template <class C, class Fn>
+__device__ __forceinline__ void for_each_min(const uint32_t* c, Fn&& fn) {
+    constexpr int W = C::W;
+    if constexpr (W == 1) {
+#pragma unroll
+        for (int j = 0; j < kStrip; ++j) fn(j, static_cast<uint32_t>(mh_at<C>(c, j)));
+    } else if constexpr (W <= 16) {
+        sliding_min<C, W, kStrip>(c, [&](int j, uint64_t v) { fn(j, static_cast<uint32_t>(v)); });
+    } else {
+        constexpr int D = W - 16;
+        uint64_t first[D];
+        sliding_min<C, 16, kStrip + D>(c, [&](int j, uint64_t v) {
+            if (j >= D) fn(j - D, static_cast<uint32_t>(min64(first[j % D], v)));
+            first[j % D] = v;
+        });
+    }
+}
+
+// for_each_min with the shard id masked to the filter's shards.
+template <class C, class Fn>
+__device__ __forceinline__ void for_each_shard(const uint32_t* c, uint32_t shard_mask, Fn&& fn) {
+    for_each_min<C>(c, [&](int j, uint32_t lo) { fn(j, lo & shard_mask); });
+}
+
+// Bit j of the result: some bit of x[j .. j + N - 1] is set (doubling spans,
+// five steps for N = 31, where a test per window cost 200 instructions a
+// strip as soon as one lane of the warp met an invalid base).
+template <int N>
+__device__ __forceinline__ uint64_t any_in_span(uint64_t x) {
+#pragma unroll
+    for (int n = 1; n < N; n += n) x |= x >> (n < N - n ? n : N - n);
+    return x;
 }
 
 // Valid-window mask: window j holds K valid bases and lies in [0, n_kmers).
-// inv[q] holds the invalid bits of code word q (bit r = base 16q + r).
+// Bit r of `bits` is set when the strip's base r is invalid.
 template <class C>
-__device__ __forceinline__ uint32_t strip_valid(const uint32_t* inv, int64_t first_kmer,
+__device__ __forceinline__ uint32_t strip_valid(uint64_t bits, int64_t first_kmer,
                                                 uint64_t n_kmers) {
     uint32_t vmask = 0xFFFFFFFFu;
-    const uint64_t bits = static_cast<uint64_t>(inv[0]) | (static_cast<uint64_t>(inv[1]) << 16) |
-                          (static_cast<uint64_t>(inv[2]) << 32) |
-                          (static_cast<uint64_t>(inv[3]) << 48);
-    constexpr uint64_t kWin = (uint64_t{1} << C::K) - 1;
-    if (bits) {
-#pragma unroll
-        for (int j = 0; j < kStrip; ++j)
-            if ((bits >> j) & kWin) vmask &= ~(1u << j);
-    }
-    if (first_kmer < 0 || first_kmer + kStrip > static_cast<int64_t>(n_kmers)) {
-#pragma unroll
-        for (int j = 0; j < kStrip; ++j) {
-            const int64_t i = first_kmer + j;
-            if (i < 0 || i >= static_cast<int64_t>(n_kmers)) vmask &= ~(1u << j);
-        }
-    }
+    if (bits) vmask = ~static_cast<uint32_t>(any_in_span<C::K>(bits));
+    const int64_t left = static_cast<int64_t>(n_kmers) - first_kmer;  // windows from the first on
+    if (first_kmer < 0) vmask = first_kmer > -kStrip ? vmask & (~0u << -first_kmer) : 0u;
+    if (left < kStrip) vmask = left > 0 ? vmask & ((1u << left) - 1u) : 0u;
     return vmask;
 }
 
@@ -370,64 +396,11 @@ __device__ __forceinline__ void insert_strip(const uint32_t* c, uint32_t vmask,
     if (prev_valid) flush(1u, prev_shard, acc);
 }
 
-// Query shard slots: the run heads of a strip fetch their 32-byte shards into
-// per-thread shared-memory slots with cp.async, all at once, so a thread has
-// every shard load of its strip in flight while it hashes the strip's s-mers.
-static_assert(kSlots * kThreads * 32 + kOverflow * kThreads * 4 == kQuerySlotBytes,
-              "slot geometry");
-
-// Half of a shard into a slot.  The .L2::64B fetch size makes an L2 miss
-// fill 64 bytes instead of 128: a random 32-byte shard then costs about 64 B
-// of DRAM reads instead of about 120 (measured with random sector reads on
-// the B200), at the same speed.
-__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src) {
-    asm volatile("cp.async.cg.shared.global.L2::64B [%0], [%1], 16;" ::"r"(smem_addr(smem_dst)),
-                 "l"(gmem_src)
-                 : "memory");
-}
 __device__ __forceinline__ void cp_async_commit() {
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() {
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-}
-
-__device__ __forceinline__ void load_shard_now(const uint64_t* p, uint64_t w[4]) {
-    asm volatile("ld.global.nc.L2::64B.v4.u64 {%0, %1, %2, %3}, [%4];"
-                 : "=l"(w[0]), "=l"(w[1]), "=l"(w[2]), "=l"(w[3])
-                 : "l"(p));
-}
-
-// The H = 4 bit addresses of the s-mer at strip position r, one per byte:
-// byte j is the bit of shard word j.
-template <class C>
-__device__ __forceinline__ uint32_t smer_bytes4(const uint32_t* c, int r) {
-    const uint64_t h = smer_hash(smer_at<C>(c, r));
-    const uint32_t lo = static_cast<uint32_t>(h), hi = static_cast<uint32_t>(h >> 32);
-    // lo bits 0-5 -> word 0, lo bits 16-21 -> word 1, hi bits 0-5 -> word 2,
-    // hi bits 16-21 -> word 3.
-    const uint32_t a = lo & 0x003F003Fu;           // b0 in byte 0, b1 in byte 2
-    const uint32_t b = (hi & 0x003F003Fu) << 8;    // b2 in byte 1, b3 in byte 3
-    return __byte_perm(a | b, 0u, 0x3120u);        // bytes b0 b1 b2 b3
-}
-
-// The same four bit addresses, one per word: b[j] is the bit of shard word j.
-template <class C>
-__device__ __forceinline__ void smer_addr4(const uint32_t* c, int r, uint32_t b[4]) {
-    const uint64_t h = smer_hash(smer_at<C>(c, r));
-    const uint32_t lo = static_cast<uint32_t>(h), hi = static_cast<uint32_t>(h >> 32);
-    b[0] = lo & 63u;
-    b[1] = (lo >> 16) & 63u;
-    b[2] = hi & 63u;
-    b[3] = (hi >> 16) & 63u;
-}
-
-template <class C>
-__device__ __forceinline__ uint32_t smer_present_h(uint64_t h, const uint64_t* w) {
-    uint32_t acc = 0xFFFFFFFFu;
-#pragma unroll
-    for (int j = 0; j < C::H; ++j) acc &= static_cast<uint32_t>(w[j & 3] >> bit_address<C::H>(h, j));
-    return acc;
 }
 
 __device__ __forceinline__ void store_strip_bytes(uint32_t result, uint8_t* out, int64_t first_kmer,
@@ -455,225 +428,416 @@ __device__ __forceinline__ void store_strip_bytes(uint32_t result, uint8_t* out,
     }
 }
 
-// Loads shard slot words x[0..7] from shared address `addr` when `pred` is
-// non-zero and leaves them unchanged otherwise: a predicated load, so a run
-// head costs no branch in the per-window loop.
-__device__ __forceinline__ void lds_slot_if(uint32_t pred, uint32_t addr, uint32_t (&x)[8]) {
+// Loads a slot's shard words x[0..7] from shared address `addr` when `pred` is
+// non-zero, leaves them unchanged otherwise, and advances `addr` to the next
+// slot after a load: predicated, so that a run head costs no branch.
+__device__ __forceinline__ void next_slot_if(uint32_t pred, uint32_t& addr, uint32_t (&x)[8]) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %8, 0;\n\t"
-        "@p ld.shared.v4.u32 {%0, %1, %2, %3}, [%9];\n\t"
-        "@p ld.shared.v4.u32 {%4, %5, %6, %7}, [%9+16];\n\t}"
+        "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %9, 0;\n\t"
+        "@p ld.shared.v4.u32 {%0, %1, %2, %3}, [%8];\n\t"
+        "@p ld.shared.v4.u32 {%4, %5, %6, %7}, [%8+16];\n\t"
+        "@p add.u32 %8, %8, 32;\n\t}"
         : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3]), "+r"(x[4]), "+r"(x[5]), "+r"(x[6]),
-          "+r"(x[7])
-        : "r"(pred), "r"(addr));
+          "+r"(x[7]), "+r"(addr)
+        : "r"(pred));
 }
 
-// Query of one strip without slots: each run head loads its shard when it is
-// reached.  Used for strips with more run heads than slots.
-template <class C>
-__device__ __noinline__ uint32_t query_strip_direct(const uint32_t* c, uint32_t vmask,
-                                                    uint32_t shard_mask, const uint64_t* words) {
-    constexpr int F = C::F;
-    uint64_t ring[F];
+// The strip's code words from shared address `at` (8-byte aligned).
+__device__ __forceinline__ void load_code_words(uint32_t at, uint32_t (&c)[kStripWords]) {
+    static_assert(kStripWords == 4, "two 8-byte loads");
+    asm volatile(
+        "ld.shared.v2.u32 {%0, %1}, [%4];\n\tld.shared.v2.u32 {%2, %3}, [%4+8];"
+        : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
+        : "r"(at)
+        : "memory");
+}
+
+// ---------------------------------------------------------------------------
+// Query of one strip
+// ---------------------------------------------------------------------------
+
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
+    uint32_t d;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
+    return d;
+}
+
+// (a & ~m) | (b & m) as one instruction (written in C it took two with a
+// constant m, 15% of the test pass).
+__device__ __forceinline__ uint32_t bit_select(uint32_t a, uint32_t b, uint32_t m) {
+    uint32_t d;
+    asm("lop3.b32 %0, %1, %2, %3, 0xD8;" : "=r"(d) : "r"(a), "r"(b), "r"(m));
+    return d;
+}
+
+// Appends `lo` to the strip's run list at shared address `at` (entries are a
+// warp's 128 bytes apart) when it differs
+// from `prev`, and sets `bit` in `chg`: predicated, since some lane of a warp
+// starts a run on almost every window.
+__device__ __forceinline__ void run_list_put(uint32_t lo, uint32_t prev, uint32_t bit,
+                                             uint32_t& at, uint32_t& chg) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, %3;\n\t"
+        "@p st.shared.u32 [%0], %2;\n\t"
+        "@p add.u32 %0, %0, 128;\n\t"
+        "@p or.b32 %1, %1, %4;\n\t}"
+        : "+r"(at), "+r"(chg)
+        : "r"(lo), "r"(prev), "r"(bit)
+        : "memory");
+}
+
+// Copies a word of shared memory when `pred` is non-zero.
+__device__ __forceinline__ void copy_u32_if(uint32_t pred, uint32_t dst, uint32_t src) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b32 v;\n\tsetp.ne.u32 p, %0, 0;\n\t"
+        "@p ld.shared.u32 v, [%2];\n\t@p st.shared.u32 [%1], v;\n\t}" ::"r"(pred),
+        "r"(dst), "r"(src)
+        : "memory");
+}
+
+// Copies the shards of slots e = lane / 2, lane / 2 + 16, ... below `total`
+// into the pool, a lane pair per slot: its two 16-byte copies go out in one
+// instruction and make one 32-byte request (a lane that issued both made two,
+// and the memory serves requests: 18.5 against 36.9 G shards/s on an 8 GiB
+// table).  An L2 miss fills 64 bytes (.L2::64B) instead of 128.
+__device__ __forceinline__ void copy_shards(uint32_t total, uint32_t pool, uint32_t ids,
+                                            uint32_t shard_mask, const uint64_t* words) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t* half = words + 2 * (lane & 1u);
+    uint32_t id = ids + 4 * (lane >> 1), dst = pool + 16 * lane;
+    for (uint32_t e = lane >> 1; __any_sync(0xFFFFFFFFu, e < total); e += 64) {
 #pragma unroll
-    for (int o = 0; o < F - 1; ++o) ring[o] = smer_hash(smer_at<C>(c, o));
-    uint64_t w[4] = {0, 0, 0, 0};
+        for (int u = 0; u < 4; ++u)
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t.reg .b32 s;\n\t.reg .b64 a;\n\t"
+                "setp.lt.u32 p, %0, %1;\n\t"
+                "@p ld.shared.u32 s, [%2];\n\t"
+                "@p and.b32 s, s, %3;\n\t"
+                "@p mad.wide.u32 a, s, 32, %4;\n\t"
+                "@p cp.async.cg.shared.global.L2::64B [%5], [a], 16;\n\t}" ::"r"(e + 16 * u),
+                "r"(total), "r"(id + 64 * u), "r"(shard_mask), "l"(half), "r"(dst + 512 * u)
+                : "memory");
+        id += 256;
+        dst += 2048;
+    }
+    cp_async_commit();
+}
+
+// Windows of one turn of the test pass.  The ring of a window's F s-mers keeps
+// position r at index r % F of the turn; turn() renames it for the next one.
+constexpr int kTurn = 16;
+static_assert(kStrip == 2 * kTurn, "two turns of one code word each");
+
+// Findere test of the window's F s-mers (F = 3 or 4) with byte permutes.  A bit
+// address is a byte n (upper three bits) and a bit t in it: for each shard
+// word one permute picks the F bytes that the s-mers name and one picks the F
+// one-bit masks, and an s-mer is missing when a mask bit is not set in its
+// byte.  With four hashes that is 8 permutes and 4 logic operations a window,
+// where F * 4 shifts of 64-bit words and their AND took 24; further sets of
+// four hashes cost the same again.  n[g][i] holds the n of set g for two words
+// in its halves, one nibble per s-mer of the window, t[g][i] the t.
+template <int F, int H>
+struct ByteTest {
+    static constexpr int kSets = H / 4;
+    // Nibble 8 reads the sign of mask byte 0, which is 0: no test.
+    static constexpr uint32_t kUnused = F == 4 ? 0u : 0x80008000u;
+    uint32_t n[kSets][2], t[kSets][2];
+
+    __device__ __forceinline__ ByteTest() {
+#pragma unroll
+        for (int g = 0; g < kSets; ++g) {
+            n[g][0] = n[g][1] = 0;
+            t[g][0] = t[g][1] = kUnused;
+        }
+    }
+    // The shard word whose hashes are in half `half` of n[g][i].
+    __device__ __forceinline__ static constexpr int word(int i, int half) {
+        return H == 8 ? i + 2 * half : 2 * i + half;
+    }
+    __device__ __forceinline__ void enter(int r, uint64_t h) {
+        const uint32_t lo = static_cast<uint32_t>(h), hi = static_cast<uint32_t>(h >> 32);
+        const int s = 4 * (r % F);
+        const uint32_t m = 0x00070007u << s;
+#pragma unroll
+        for (int g = 0; g < kSets; ++g) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                // Bit addresses at bits 0-5 and 16-21 (other bits are ignored).
+                uint32_t a;
+                if constexpr (H == 4)
+                    a = i ? hi : lo;
+                else if constexpr (H == 8)
+                    a = (g ? hi : lo) >> (8 * i);
+                else
+                    a = bit_address<H>(h, 4 * g + 2 * i) | (bit_address<H>(h, 4 * g + 2 * i + 1) << 16);
+                n[g][i] = bit_select(n[g][i], s ? a << (s ? s - 3 : 0) : a >> 3, m);
+                t[g][i] = bit_select(t[g][i], a << s, m);
+            }
+        }
+    }
+    // Non-zero when an s-mer of the window is missing from shard x.
+    __device__ __forceinline__ uint32_t missing(const uint32_t (&x)[8]) const {
+        uint32_t bad = 0;
+#pragma unroll
+        for (int g = 0; g < kSets; ++g) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    const int q = word(i, half);
+                    bad |= prmt(0x08040201u, 0x80402010u, t[g][i] >> (16 * half)) &
+                           ~prmt(x[2 * q], x[2 * q + 1], n[g][i] >> (16 * half));
+                }
+            }
+        }
+        return bad;
+    }
+    __device__ __forceinline__ void turn() {
+        if constexpr (F == 3) {  // index i takes over from (i + 16) % 3
+            auto rotate = [](uint32_t v) {
+                return ((v >> 4) & 0x00FF00FFu) | ((v & 0x000F000Fu) << 8);
+            };
+#pragma unroll
+            for (int g = 0; g < kSets; ++g) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    n[g][i] = rotate(n[g][i]);
+                    t[g][i] = rotate(t[g][i]) | kUnused;
+                }
+            }
+        }
+    }
+};
+
+// The word `q` of shard x shifted down by `b`: bit b in bit 0.
+__device__ __forceinline__ uint32_t shard_bit(const uint32_t (&x)[8], int q, uint32_t b) {
+    return static_cast<uint32_t>(((static_cast<uint64_t>(x[2 * q + 1]) << 32) | x[2 * q]) >> b);
+}
+
+// The same test by shifts of 64-bit words, for four hashes and other F.
+template <int F>
+struct ShiftTest {
+    uint32_t b[F][4];
+
+    __device__ __forceinline__ void enter(int r, uint64_t h) {
+        const uint32_t lo = static_cast<uint32_t>(h), hi = static_cast<uint32_t>(h >> 32);
+        b[r % F][0] = lo & 63u;
+        b[r % F][1] = (lo >> 16) & 63u;
+        b[r % F][2] = hi & 63u;
+        b[r % F][3] = (hi >> 16) & 63u;
+    }
+    __device__ __forceinline__ uint32_t missing(const uint32_t (&x)[8]) const {
+        uint32_t present = 1u;
+#pragma unroll
+        for (int o = 0; o < F; ++o) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) present &= shard_bit(x, q, b[o][q]);
+        }
+        return ~present & 1u;
+    }
+    __device__ __forceinline__ void turn() {
+        const ShiftTest old = *this;
+#pragma unroll
+        for (int i = 0; i < F; ++i) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) b[i][q] = old.b[(i + kTurn) % F][q];
+        }
+    }
+};
+
+// The same test from a ring of hashes, for H hashes or long rings.
+template <int F, int H>
+struct HashTest {
+    uint64_t h[F];
+
+    __device__ __forceinline__ void enter(int r, uint64_t v) { h[r % F] = v; }
+    __device__ __forceinline__ uint32_t missing(const uint32_t (&x)[8]) const {
+        uint32_t present = 1u;
+#pragma unroll
+        for (int o = 0; o < F; ++o) {
+#pragma unroll
+            for (int j = 0; j < H; ++j) present &= shard_bit(x, j & 3, bit_address<H>(h[o], j));
+        }
+        return ~present & 1u;
+    }
+    __device__ __forceinline__ void turn() {
+        const HashTest old = *this;
+#pragma unroll
+        for (int i = 0; i < F; ++i) h[i] = old.h[(i + kTurn) % F];
+    }
+};
+
+template <class C, int kKind = (C::F == 3 || C::F == 4) ? 0 : (C::H == 4 && C::F <= 8) ? 1 : 2>
+struct FindereTest {
+    using type = HashTest<C::F, C::H>;
+};
+template <class C>
+struct FindereTest<C, 0> {
+    using type = ByteTest<C::F, C::H>;
+};
+template <class C>
+struct FindereTest<C, 1> {
+    using type = ShiftTest<C::F>;
+};
+
+// The minimizer pass of a strip: lists its runs (one low hash word per run)
+// from shared address `list` on.  Returns the windows that start a run
+// (x) and the low hash words of window 0 and window 31 (y, z).  A function of
+// its own, so that its registers (two 64-bit arrays of W) do not add to the
+// kernel's.
+template <class C>
+__device__ __noinline__ uint3 list_runs(uint32_t code_mem, uint32_t list) {
+    uint32_t c[kStripWords];
+    load_code_words(code_mem, c);
+    uint32_t at = list, chg = 1u, first = 0, prev = 0;
+    for_each_min<C>(c, [&](int j, uint32_t lo) {
+        if (j == 0) {
+            asm volatile("st.shared.u32 [%0], %1;" ::"r"(at), "r"(lo) : "memory");
+            at += 128;
+            first = lo;
+        } else {
+            run_list_put(lo, prev, 1u << j, at, chg);
+        }
+        prev = lo;
+    });
+    return make_uint3(chg, first, prev);
+}
+
+// Query of one strip: the minimizer pass lists the strip's runs, the runs that
+// hold a valid window get consecutive slots of the warp's pool (a prefix sum
+// over the lanes), the warp copies their shards there, and the test pass
+// walks the windows with the current run's shard in registers.  Window 0's
+// run reads the left lane's last slot, the one before the lane's own, when
+// that lane's last run continues into the strip.  Lanes whose runs do not fit
+// the pool any more wait for another round.
+//
+// Bound: the integer logic pipe (72% busy on <31,28,16,4>), then the latency
+// of the shard copies.  1.51e9 positions of 10 M reads against 8 GiB: 5.95 ms,
+// 25 G shards/s; with the copies issued by the thread that finds a run (two
+// requests per shard), a copy slot per thread and shifts for the bit tests it
+// was 7.82 ms at 19 G shards/s, the rate at which the memory takes two 16-byte
+// requests each.  Loading the shards to registers instead keeps the L1 lines
+// of all requests in flight and was slower with every byte of shared memory
+// in use (6.8 ms at 150 KB an SM, 8.6 at 203 KB).
+template <class C>
+__device__ __forceinline__ uint32_t query_strip(uint32_t code_mem, uint32_t vmask,
+                                                uint32_t shard_mask, const uint64_t* words,
+                                                uint32_t run_mem) {
+    constexpr int F = C::F;
+    constexpr uint32_t kPoolSlots = query_pool_slots(C::W, C::H);
+    static_assert(kPoolSlots * 32 >= 32 * 128, "the run lists fit the pool");
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t result = 0;
+    while (__any_sync(0xFFFFFFFFu, vmask != 0u)) {
+        const uint32_t list = run_mem + 4 * lane;
+        const uint3 runs = list_runs<C>(code_mem, list);
+        const uint32_t chg = runs.x, first = runs.y, prev = runs.z;
+        // Run heads: a valid window whose predecessor is invalid or of another run.
+        uint32_t heads = vmask & (chg | ~(vmask << 1));
+        const int n = __popc(heads);
+        // A lane lends its last slot when that holds window 31's run and the run
+        // is not its window 0's, which may itself be borrowed.
+        const bool lend = n > 0 && (vmask >> (kStrip - 1)) && !(n == 1 && (vmask & 1u));
+        const uint32_t left_lo = __shfl_up_sync(0xFFFFFFFFu, prev, 1);
+        const uint32_t lenders = __ballot_sync(0xFFFFFFFFu, lend);
+        const bool borrow =
+            lane > 0 && (heads & 1u) && (lenders >> (lane - 1) & 1u) && left_lo == first;
+        const uint32_t own = n - (borrow ? 1 : 0);
+        uint32_t end = own;
+#pragma unroll
+        for (int o = 1; o < 32; o *= 2) {
+            const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, end, o);
+            if (lane >= static_cast<uint32_t>(o)) end += v;
+        }
+        const uint32_t begin = end - own;
+        // The lanes that fit are the first ones, so a lender fits if its borrower does.
+        const bool fits = end <= kPoolSlots;
+        if (!fits) heads = 0;
+        // The shard ids of the lane's slots, from its list: a head's entry is the
+        // number of runs that start up to it.
+        const uint32_t ids = run_mem + 32 * kPoolSlots;
+        uint32_t rest = borrow ? heads & (heads - 1u) : heads;
+        for (uint32_t at = ids + 4 * begin; __any_sync(0xFFFFFFFFu, rest != 0u); at += 4) {
+            const uint32_t b = rest & (0u - rest);
+            rest ^= b;
+            const uint32_t e = __popc(chg & (b ^ (b - 1u))) - 1;
+            copy_u32_if(b, at, list + 128 * e);
+        }
+        __syncwarp();
+        copy_shards(__reduce_max_sync(0xFFFFFFFFu, fits ? end : 0u), run_mem, ids, shard_mask,
+                    words);
+        uint32_t c[kStripWords];
+        load_code_words(code_mem, c);
+        typename FindereTest<C>::type test;
+#pragma unroll
+        for (int o = 0; o < F - 1; ++o) test.enter(o, smer_hash(smer_at<C>(c, o)));
+        cp_async_wait_all();
+        __syncwarp();
+        uint32_t x[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        uint32_t at = run_mem + 32 * (borrow ? begin - 1 : begin);
+        uint32_t missing = 0;
+        // Turns of 16 windows, the code words moving down by one: half the
+        // instructions of 32 unrolled windows, which ran out of the instruction
+        // cache (10% of the stalls).
+#pragma unroll 1
+        for (int turn = 0; turn < 2; ++turn) {
+            uint32_t m = 0;
+#pragma unroll
+            for (int j = 0; j < kTurn; ++j) {
+                test.enter(j + F - 1, smer_hash(smer_at<C>(c, j + F - 1)));
+                next_slot_if(heads & (1u << j), at, x);
+                m += min(test.missing(x), 1u) << j;
+            }
+            test.turn();
+            missing = (missing >> kTurn) | (m << kTurn);
+            heads >>= kTurn;
+            c[0] = c[1];
+            c[1] = c[2];
+            c[2] = c[3];
+        }
+        if (fits) {
+            result |= vmask & ~missing;
+            vmask = 0;
+        }
+        __syncwarp();  // borrowed slots are read before another round's lists replace them
+    }
+    return result;
+}
+
+// Query of one strip without a pool: each run head loads its shard when it is
+// reached.  For windows of less than 6 m-mers of at most 8 bases, whose runs are so short (a head
+// every second window at W = 3) that a pool would take several rounds, and
+// whose m-mers are so few that the shards stay in the caches: 100 M windows of
+// <5,4,3,4> took 0.32 ms, two rounds through the pool 1.53.
+template <class C>
+__device__ __forceinline__ uint32_t query_strip_direct(uint32_t code_mem, uint32_t vmask,
+                                                       uint32_t shard_mask,
+                                                       const uint64_t* words) {
+    constexpr int F = C::F;
+    uint32_t c[kStripWords];
+    load_code_words(code_mem, c);
+    typename FindereTest<C>::type test;
+#pragma unroll
+    for (int o = 0; o < F - 1; ++o) test.enter(o, smer_hash(smer_at<C>(c, o)));
+    uint32_t x[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    uint32_t cur = 0, missing = 0;
     bool have = false;
-    uint32_t cur = 0, result = 0;
     for_each_shard<C>(c, shard_mask, [&](int j, uint32_t sh) {
-        ring[(j + F - 1) % F] = smer_hash(smer_at<C>(c, j + F - 1));
-        const bool valid = (vmask >> j) & 1u;
-        if (valid && (!have || sh != cur)) {
-            load_shard_now(words + static_cast<uint64_t>(sh) * 4, w);
+        test.enter(j + F - 1, smer_hash(smer_at<C>(c, j + F - 1)));
+        if (((vmask >> j) & 1u) && (!have || sh != cur)) {
+            uint64_t w[4];
+            load_shard(words + static_cast<uint64_t>(sh) * 4, w[0], w[1], w[2], w[3]);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                x[2 * q] = static_cast<uint32_t>(w[q]);
+                x[2 * q + 1] = static_cast<uint32_t>(w[q] >> 32);
+            }
             cur = sh;
             have = true;
         }
-        uint32_t present = valid ? 1u : 0u;
-#pragma unroll
-        for (int o = 0; o < F; ++o) present &= smer_present_h<C>(ring[(j + o) % F], w);
-        result |= (present & 1u) << j;
+        missing |= min(test.missing(x), 1u) << j;
     });
-    return result;
-}
-
-// Query of one strip: minimizers -> cp.async of every run head's shard into
-// the thread's slots (issued as the heads are found) -> s-mer hashing while
-// the copies are in flight -> wait -> findere tests -> output bytes.
-// kAddrInLoop (four hashes): compute each position's bit addresses as it
-// enters the window instead of packing the strip's addresses while the
-// copies fly.  It frees 35 registers and makes the plain <31,28,16,4> query
-// 1.1% faster, but spills in the ragged kernels and with one s-mer per
-// window, which keep the packed form.
-template <class C, bool kAddrInLoop>
-__device__ __forceinline__ uint32_t query_strip(const uint32_t* c, uint32_t vmask, uint32_t shard_mask,
-                                            const uint64_t* words, uint64_t* slot0,
-                                            uint32_t* ovf0, uint8_t* out, int64_t first_kmer,
-                                            uint64_t n_kmers) {
-    // Slot n of this thread lives at slot0 + n * kThreads * 4 and overflow
-    // entry e at ovf0 + e * kThreads ([entry][thread] layouts: neighbouring
-    // threads touch neighbouring addresses).
-    constexpr int kSlotStride = kThreads * 4;
-    constexpr int F = C::F;
-    // Run heads: a valid window whose predecessor is invalid or selects
-    // another shard.  The first kSlots heads copy their shard into slots; the
-    // next kOverflow only record their shard id (loaded when reached).  The
-    // copy for window 0 is decided after the loop: when the left neighbour's
-    // last run continues into this strip (same shard, both ends valid), its
-    // staged slot is read instead of loading the sector again.
-    uint32_t heads = 0;
-    int n = 0;
-    uint32_t first_sh = 0, last_sh = 0;
-    {
-        uint32_t prev = 0;
-        for_each_shard<C>(c, shard_mask, [&](int j, uint32_t sh) {
-            const bool valid = (vmask >> j) & 1u;
-            const bool prev_valid = j > 0 && ((vmask >> (j - 1)) & 1u);
-            if (j == 0) first_sh = sh;
-            if (j == kStrip - 1) last_sh = sh;
-            if (valid && (!prev_valid || sh != prev)) {
-                heads |= 1u << j;
-                if (j > 0) {
-                    if (n < kSlots) {
-                        const uint64_t* src = words + static_cast<uint64_t>(sh) * 4;
-                        uint64_t* dst = slot0 + n * kSlotStride;
-                        cp_async16(dst, src);
-                        cp_async16(dst + 2, src + 2);
-                    } else if (n < kSlots + kOverflow) {
-                        ovf0[(n - kSlots) * kThreads] = sh;
-                    }
-                }
-                ++n;
-            }
-            prev = sh;
-        });
-    }
-    const int lane = threadIdx.x & 31;
-    const bool last_open = (vmask >> (kStrip - 1)) & 1u;
-    // Lend the last run's slot only when its head is not window 0: window 0's
-    // slot may itself be borrowed (never loaded), so lending it would chain.
-    const bool last_is_w0 = n == 1 && (vmask & 1u);
-    const int my_last_slot = last_open && n >= 1 && n <= kSlots && !last_is_w0 ? n - 1 : -1;
-    const uint32_t left_sh = __shfl_up_sync(0xFFFFFFFFu, last_sh, 1);
-    const int left_slot = __shfl_up_sync(0xFFFFFFFFu, my_last_slot, 1);
-    const bool borrow = lane > 0 && (vmask & 1u) && left_slot >= 0 && left_sh == first_sh;
-    if ((vmask & 1u) && !borrow) {
-        const uint64_t* src = words + static_cast<uint64_t>(first_sh) * 4;
-        cp_async16(slot0, src);
-        cp_async16(slot0 + 2, src + 2);
-    }
-    cp_async_commit();
-    if (n > kSlots + kOverflow) {
-        cp_async_wait_all();
-        __syncwarp();
-        const uint32_t direct = query_strip_direct<C>(c, vmask, shard_mask, words);
-        if (out) store_strip_bytes(direct, out, first_kmer, n_kmers);
-        return direct;
-    }
-    // Hash the strip's s-mers while the shard copies are in flight (with
-    // four hashes, one word of bit addresses per position), unless
-    // kAddrInLoop computes them as the positions enter the window.
-    constexpr int NP = kStrip + F - 1;
-    constexpr bool kPacked = C::H == 4 && !kAddrInLoop;
-    uint32_t bytes[kPacked ? NP : 1];
-    uint64_t hs[C::H == 4 ? 1 : NP];
-#pragma unroll
-    for (int r = 0; r < NP; ++r) {
-        if constexpr (kPacked)
-            bytes[r] = smer_bytes4<C>(c, r);
-        else if constexpr (C::H != 4)
-            hs[r] = smer_hash(smer_at<C>(c, r));
-    }
-    cp_async_wait_all();
-    __syncwarp();  // neighbours' slots are complete before any is borrowed
-    uint64_t w[4] = {0, 0, 0, 0};
-    uint32_t result = 0;
-    // Bit addresses of the F positions of the current window, extracted once
-    // per position as it enters the window.
-    uint32_t ring[C::H == 4 ? F : 1][4];
-    auto enter = [&](int r) {  // position r enters the window
-        if constexpr (kPacked) {
-#pragma unroll
-            for (int q = 0; q < 4; ++q) ring[r % F][q] = __byte_perm(bytes[r], 0u, 0x4440u + q);
-        } else if constexpr (C::H == 4) {
-            smer_addr4<C>(c, r, ring[r % F]);
-        }
-    };
-#pragma unroll
-    for (int o = 0; o < F - 1; ++o) enter(o);
-    // (Configurations with one s-mer per window or sixteen hashes keep the
-    // branching loop below: the predicated form spills registers there.)
-    constexpr bool kPredicated = F > 1 && C::H <= 8;
-    if (kPredicated && n <= kSlots) {
-        // Every head's shard is in a slot (the common case): each window
-        // does a predicated load of the next head's slot and advances the
-        // slot address when it is a head, so the loop has no per-head branch.
-        const uint64_t* sfirst = borrow ? slot0 + left_slot * kSlotStride - 4 : slot0;
-        uint32_t addr = smem_addr(sfirst);
-        const uint32_t base = smem_addr(slot0);
-        uint32_t x[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        uint32_t loaded = 0;
-#pragma unroll
-        for (int j = 0; j < kStrip; ++j) {
-            enter(j + F - 1);
-            const uint32_t head = (heads >> j) & 1u;
-            lds_slot_if(head, addr, x);
-            loaded += head;
-            addr = head ? base + loaded * (kSlotStride * 8) : addr;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) w[q] = (static_cast<uint64_t>(x[2 * q + 1]) << 32) | x[2 * q];
-            uint32_t present = (vmask >> j) & 1u;
-#pragma unroll
-            for (int o = 0; o < F; ++o) {
-                if constexpr (C::H == 4) {
-                    const uint32_t* b = ring[(j + o) % F];
-                    present &= static_cast<uint32_t>(w[0] >> b[0]) & static_cast<uint32_t>(w[1] >> b[1]) &
-                               static_cast<uint32_t>(w[2] >> b[2]) & static_cast<uint32_t>(w[3] >> b[3]);
-                } else {
-                    present &= smer_present_h<C>(hs[j + o], w);
-                }
-            }
-            result |= (present & 1u) << j;
-        }
-        if (out) store_strip_bytes(result, out, first_kmer, n_kmers);
-        return result;
-    }
-    // More heads than slots: the later heads load their shards directly.
-    n = 0;
-#pragma unroll
-    for (int j = 0; j < kStrip; ++j) {
-        enter(j + F - 1);
-        if ((heads >> j) & 1u) {
-            if (n < kSlots) {
-                // Slot 0 may be the left neighbour's last slot (its thread's
-                // slots sit 4 words below this thread's).
-                const uint64_t* sn = (n == 0 && borrow) ? slot0 + left_slot * kSlotStride - 4
-                                                        : slot0 + n * kSlotStride;
-                const uint4 lo = *reinterpret_cast<const uint4*>(sn);
-                const uint4 hi = *reinterpret_cast<const uint4*>(sn + 2);
-                w[0] = (static_cast<uint64_t>(lo.y) << 32) | lo.x;
-                w[1] = (static_cast<uint64_t>(lo.w) << 32) | lo.z;
-                w[2] = (static_cast<uint64_t>(hi.y) << 32) | hi.x;
-                w[3] = (static_cast<uint64_t>(hi.w) << 32) | hi.z;
-            } else {
-                load_shard_now(words + static_cast<uint64_t>(ovf0[(n - kSlots) * kThreads]) * 4, w);
-            }
-            ++n;
-        }
-        uint32_t present = (vmask >> j) & 1u;
-#pragma unroll
-        for (int o = 0; o < F; ++o) {
-            if constexpr (C::H == 4) {
-                const uint32_t* b = ring[(j + o) % F];
-                present &= static_cast<uint32_t>(w[0] >> b[0]) & static_cast<uint32_t>(w[1] >> b[1]) &
-                           static_cast<uint32_t>(w[2] >> b[2]) & static_cast<uint32_t>(w[3] >> b[3]);
-            } else {
-                present &= smer_present_h<C>(hs[j + o], w);
-            }
-        }
-        result |= (present & 1u) << j;
-    }
-    if (out) store_strip_bytes(result, out, first_kmer, n_kmers);
-    return result;
+    return vmask & ~missing;
 }
 
 // ---------------------------------------------------------------------------
@@ -681,7 +845,7 @@ __device__ __forceinline__ uint32_t query_strip(const uint32_t* c, uint32_t vmas
 // ---------------------------------------------------------------------------
 
 // Ragged launches: marks the record structure of the staged tile.  brk bit
-// r of word q is set when tile position 16q + r starts a record (windows
+// r of word q is set when tile position 32q + r starts a record (windows
 // that contain it and the byte before it span two records); bytes outside
 // every record are added to the invalid bits.  Each thread takes records
 // first, first + kThreads, ... of those overlapping the tile.
@@ -698,7 +862,7 @@ __device__ __forceinline__ void mark_records(const TileParams& p, int64_t s0, ui
             const int64_t pos = x - s0;
             const int q = static_cast<int>(pos >> 4), r = static_cast<int>(pos & 15);
             const int64_t n = (16 - r) < (b - x) ? (16 - r) : (b - x);
-            atomicOr(arr + q, ((1u << n) - 1u) << r);
+            atomicOr(arr + (q >> 1), ((1u << n) - 1u) << (r + 16 * (q & 1)));
             x += n;
         }
     };
@@ -718,7 +882,7 @@ __device__ __forceinline__ void mark_records(const TileParams& p, int64_t s0, ui
         const int64_t b = a + static_cast<int64_t>(rec.bytes);
         if (a > s0 && a < t_end) {
             const int64_t pos = a - s0;
-            atomicOr(brk + (pos >> 4), 1u << (pos & 15));
+            atomicOr(brk + (pos >> 5), 1u << (pos & 31));
         }
         const int64_t next = r + 1 < n ? static_cast<int64_t>(p.ranges[r + 1].offset) : len;
         if (next > b) set_bits(inval, b, next);
@@ -726,17 +890,11 @@ __device__ __forceinline__ void mark_records(const TileParams& p, int64_t s0, ui
 }
 
 // Ragged launches: clears windows j of the strip that contain a record start
-// other than their own first byte.
+// other than their own first byte.  Bit r of `bits`: a record starts at base r.
 template <class C>
-__device__ __forceinline__ uint32_t strip_in_record(const uint32_t* bk, uint32_t vmask) {
-    const uint64_t bits = static_cast<uint64_t>(bk[0]) | (static_cast<uint64_t>(bk[1]) << 16) |
-                          (static_cast<uint64_t>(bk[2]) << 32) |
-                          (static_cast<uint64_t>(bk[3]) << 48);
-    constexpr uint64_t kInner = ((uint64_t{1} << C::K) - 1) >> 1;  // positions j+1 .. j+K-1
-    if (bits) {
-#pragma unroll
-        for (int j = 0; j < kStrip; ++j)
-            if ((bits >> (j + 1)) & kInner) vmask &= ~(1u << j);
+__device__ __forceinline__ uint32_t strip_in_record(uint64_t bits, uint32_t vmask) {
+    if constexpr (C::K > 1) {
+        if (bits) vmask &= ~static_cast<uint32_t>(any_in_span<C::K - 1>(bits >> 1));
     }
     return vmask;
 }
@@ -813,18 +971,21 @@ __device__ __forceinline__ void tally_records(const TileParams& p, uint32_t firs
 // Persistent tile kernel.  Plain launches walk tiles blockIdx.x + i * gridDim.x;
 // ragged launches take tiles from the device work-queue counter p.queue, so
 // tiles of uneven cost (records of any length, N runs) balance across CTAs.
-// Either way tile i+2 is known while tile i is processed, so its staging copy
-// is issued two tiles ahead.
+// Either way tile i+2 is taken while tile i is processed, and tile i+1's
+// staging copy is issued once tile i's bytes are encoded, into the same buffer.
 template <class C, bool kQuery, bool kDense, bool kRagged>
-__global__ void __launch_bounds__(kThreads, 2) tile_kernel(TileParams p) {
-    __shared__ alignas(128) uint8_t stage[2][kStageBytes];
-    __shared__ uint32_t code[kCodeWords + 4];
-    __shared__ uint32_t inval[kCodeWords + 4];
-    __shared__ uint32_t brk[kRagged ? kCodeWords + 4 : 1];
+__global__ void __launch_bounds__(kThreads, kQuery && query_three_ctas(C::W, C::H) ? 3 : 2)
+    tile_kernel(TileParams p) {
+    __shared__ alignas(128) uint8_t stage[kStageBytes];
+    __shared__ alignas(8) uint32_t code[kCodeWords + 4];
+    // One bit per position: invalid bases, record starts.
+    __shared__ alignas(8) uint32_t inval[kCodeWords / 2 + 1];
+    __shared__ alignas(8) uint32_t brk[kRagged ? kCodeWords / 2 + 1 : 1];
     __shared__ uint64_t tiles[3];
     __shared__ uint32_t first_rec[3];
     __shared__ unsigned long long tally[2];
-    __shared__ alignas(8) uint64_t bars[2];
+    __shared__ bool covered;  // the staged tile needs no plain loads
+    __shared__ alignas(8) uint64_t bar;
     __shared__ uint64_t onehot[kQuery ? 1 : 64];
 
     const int tid = threadIdx.x;
@@ -850,85 +1011,88 @@ __global__ void __launch_bounds__(kThreads, 2) tile_kernel(TileParams p) {
         return t;
     };
     if (tid == 0) {
-        mbar_init(&bars[0], 1);
-        mbar_init(&bars[1], 1);
+        mbar_init(&bar, 1);
         mbar_fence_init();
         tally[0] = tally[1] = 0;
-        const uint64_t t0 = take(0, 0), t1 = take(1, 1);
-        if (t0 < p.n_tiles) issue_stage<kDense>(p, t0, stage[0], &bars[0]);
-        if (t1 < p.n_tiles) issue_stage<kDense>(p, t1, stage[1], &bars[1]);
+        const uint64_t t0 = take(0, 0);
+        take(1, 1);
+        if (t0 < p.n_tiles) covered = issue_stage<kDense>(p, t0, stage, &bar);
     }
     __syncthreads();
-    // Dynamic shared memory, [slot][thread] layout: the query kernel's shard
-    // slots (kQuerySlotBytes per CTA) or the insert kernel's flush staging
-    // ring (kInsertSlotBytes per CTA).
+    // Dynamic shared memory: the query kernel's pool of shard slots, a part per
+    // warp (query_cta_bytes per CTA), or the insert kernel's flush staging ring,
+    // [slot][thread] (kInsertSlotBytes per CTA).
     extern __shared__ __align__(16) uint64_t slots[];
     FlushRing ring{slots + 4 * tid, 0u};
     (void)ring;
     unsigned long long n_valid = 0, n_pos = 0;
+    const uint32_t origin = stage_origin<kDense>(p);
     for (uint32_t it = 0;; ++it) {
         const uint64_t tile = tiles[it % 3];
         if (tile >= p.n_tiles) break;
-        const int b = it & 1;
-        const uint32_t parity = (it >> 1) & 1u;
-        const bool ok = mbar_wait_bounded(&bars[b], parity);
+        const bool ok = mbar_wait_bounded(&bar, it & 1u);
         if (__syncthreads_or(!ok)) {
-            // Both staging buffers may still have a bulk copy in flight:
-            // this tile's (whose wait ran out) and the next tile's.  Give
-            // each one more bounded wait before the CTA's shared memory is
-            // released, so no copy lands in memory a later CTA owns.
+            // The copy that ran out of time may still be in flight: give it
+            // one more bounded wait before the CTA's shared memory is
+            // released, so that it does not land in memory a later CTA owns.
             if (tid == 0) {
                 atomicExch(p.err, kDevErrStageTimeout);
-                (void)mbar_wait_bounded(&bars[b], parity);
-                if (tiles[(it + 1) % 3] < p.n_tiles)
-                    (void)mbar_wait_bounded(&bars[b ^ 1], ((it + 1) >> 1) & 1u);
+                (void)mbar_wait_bounded(&bar, it & 1u);
             }
             __syncthreads();
             if constexpr (!kQuery) flush_ring_drain();
             return;
         }
-        const TileGeom g = tile_geom<kDense>(p, tile);
-        fill_ragged<kDense>(p, g, stage[b]);
-        __syncthreads();
+        if (!covered) {
+            fill_ragged<kDense>(p, tile_geom<kDense>(p, tile), stage);
+            __syncthreads();
+        }
+        const int64_t s0 = tile_first_symbol(p, tile);
         for (int q = tid; q < kCodeWords; q += kThreads) {
             uint32_t cw, iv;
-            encode_word<kDense>(g, stage[b], q, cw, iv);
+            encode_word<kDense>(origin, stage, q, cw, iv);
             code[q] = cw;
-            inval[q] = iv;
-            if constexpr (kRagged) brk[q] = 0u;
+            reinterpret_cast<uint16_t*>(inval)[q] = static_cast<uint16_t>(iv);
+            if constexpr (kRagged) reinterpret_cast<uint16_t*>(brk)[q] = 0;
         }
         if constexpr (kRagged) {
             __syncthreads();
-            mark_records<C>(p, g.s0, first_rec[it % 3], inval, brk);
+            mark_records<C>(p, s0, first_rec[it % 3], inval, brk);
         }
         __syncthreads();
         if (tid == 0) {
-            const uint64_t t2 = take(it + 2, (it + 2) % 3);
-            if (t2 < p.n_tiles) issue_stage<kDense>(p, t2, stage[b], &bars[b]);
+            // The staged bytes are encoded: the next tile's copy goes out and
+            // lands while this one is hashed.  The tile after it is taken now,
+            // so that a barrier lies between its slot's write and its reads.
+            const uint64_t next = tiles[(it + 1) % 3];
+            if (next < p.n_tiles) covered = issue_stage<kDense>(p, next, stage, &bar);
+            take(it + 2, (it + 2) % 3);
         }
 
-        uint32_t c[kStripWords], iv[kStripWords];
+        uint32_t c[kStripWords];
 #pragma unroll
-        for (int q = 0; q < kStripWords; ++q) {
-            c[q] = code[tid * (kStrip / 16) + q];
-            iv[q] = inval[tid * (kStrip / 16) + q];
-        }
-        const int64_t first_kmer = g.s0 + static_cast<int64_t>(tid) * kStrip;
-        uint32_t vmask = strip_valid<C>(iv, first_kmer, p.n_kmers);
+        for (int q = 0; q < kStripWords; ++q) c[q] = code[tid * (kStrip / 16) + q];
+        static_assert(kStrip == 32 && kStripWords == 4, "a strip's bits are two 32-bit words");
+        auto strip_bits = [&](const uint32_t* a) {
+            return static_cast<uint64_t>(a[tid]) | (static_cast<uint64_t>(a[tid + 1]) << 32);
+        };
+        const int64_t first_kmer = s0 + static_cast<int64_t>(tid) * kStrip;
+        uint32_t vmask = strip_valid<C>(strip_bits(inval), first_kmer, p.n_kmers);
         if constexpr (kRagged) {
-            uint32_t bk[kStripWords];
-#pragma unroll
-            for (int q = 0; q < kStripWords; ++q) bk[q] = brk[tid * (kStrip / 16) + q];
-            vmask = strip_in_record<C>(bk, vmask);
+            vmask = strip_in_record<C>(strip_bits(brk), vmask);
             n_valid += __popc(vmask);
         }
         uint32_t hits = 0;
         if constexpr (kQuery) {
-            constexpr bool kAddrInLoop = !kRagged && C::W == 16 && C::F > 1;
-            hits = query_strip<C, kAddrInLoop>(
-                c, vmask, p.shard_mask, p.words, slots + 4 * tid,
-                reinterpret_cast<uint32_t*>(slots + kSlots * kThreads * 4) + tid, p.out,
-                first_kmer, p.n_kmers);
+            const uint32_t code_mem = smem_addr(code + tid * (kStrip / 16));
+            if constexpr (C::W < 6 && C::M <= 8) {
+                hits = query_strip_direct<C>(code_mem, vmask, p.shard_mask, p.words);
+            } else {
+                constexpr int kWarpBytes = query_warp_bytes(C::W, C::H);
+                hits = query_strip<C>(code_mem, vmask, p.shard_mask, p.words,
+                                      smem_addr(slots) + (tid >> 5) * kWarpBytes);
+            }
+            if (p.out) store_strip_bytes(hits, p.out, first_kmer, p.n_kmers);
             if constexpr (kRagged) n_pos += __popc(hits & vmask);
             // Bit-packed mode (grid phase 0, so strips start at multiples of
             // 32 windows): one 32-bit word per strip, coalesced across the warp.
