@@ -17,7 +17,7 @@ constexpr int kStripWords = kStrip / 16 + 2;           // code words one strip r
 constexpr int kCodeWords = (kThreads - 1) * (kStrip / 16) + kStripWords;  // per tile
 constexpr int kStageBytes = kCodeWords * 16 + 64;      // staged input bytes per buffer
 constexpr int kFlushSlots = 8;                         // insert bulk-reduce staging slots
-constexpr int kInsertSlotBytes = kFlushSlots * kThreads * 32;  // dynamic smem of inserts
+constexpr int kInsertSlotBytes = kFlushSlots * kThreads * 32;  // dynamic smem of flush rings
 
 // A warp's dynamic shared memory in the query kernels: a pool of shard slots
 // (first the run lists of its lanes, 32 entries each) and the shard id of
@@ -37,6 +37,16 @@ SBF_SIZE_FN bool query_three_ctas(int w, int h) { return w >= 10 && w <= 16 && h
 SBF_SIZE_FN int query_pool_slots(int w, int h) { return query_three_ctas(w, h) ? 208 : 344; }
 SBF_SIZE_FN int query_warp_bytes(int w, int h) { return query_pool_slots(w, h) * (32 + 4); }
 SBF_SIZE_FN int query_cta_bytes(int w, int h) { return kThreads / 32 * query_warp_bytes(w, h); }
+
+// The insert kernels' part of a warp: the same pool, filled with the runs' word
+// masks, and a spare slot per lane for a run that a neighbour flushes.  184
+// slots leave room for three CTAs and 4 deviations at W = 12 (158 slots).
+SBF_SIZE_FN bool insert_three_ctas(int w, int h) { return w >= 12 && w <= 16 && h <= 8; }
+SBF_SIZE_FN int insert_pool_slots(int w, int h) { return insert_three_ctas(w, h) ? 184 : 320; }
+SBF_SIZE_FN int insert_warp_bytes(int w, int h) {
+    return insert_pool_slots(w, h) * (32 + 4) + 32 * 32;
+}
+SBF_SIZE_FN int insert_cta_bytes(int w, int h) { return kThreads / 32 * insert_warp_bytes(w, h); }
 
 // A record of a ragged launch: bytes [offset, offset + bytes) of the input.
 // Same layout as sbf_record_range of the C ABI.
@@ -120,7 +130,7 @@ struct KernelSet {
     const void* query_ragged;
     // Dynamic shared memory of the insert and query kernels: the tile
     // kernels' flush ring and shard pool; none for the generic kernels.
-    int smem_insert = kInsertSlotBytes;
+    int smem_insert = insert_cta_bytes(k - m + 1, h);
     int smem_query = query_cta_bytes(k - m + 1, h);
     bool jit = false;    // loaded from a run-time compiled library
     int jit_occupancy = 2;  // resident CTAs per SM assumed for run-time compiled sets

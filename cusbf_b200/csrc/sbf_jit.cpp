@@ -312,6 +312,7 @@ const KernelSet* jit_kernels(int k, int s, int m, int h, int alphabet, int devic
         if (!jc.tile()) {
             // The generic kernels use few registers; inserts take the flush
             // ring's dynamic shared memory, queries none.
+            e->ks.smem_insert = kInsertSlotBytes;
             e->ks.smem_query = 0;
             e->ks.jit_occupancy = 4;
         }

@@ -15,6 +15,7 @@
 #include <cstdint>
 
 #include "../../include/sbf_b200.h"
+#include "sbf_flush.cuh"
 #include "sbf_host.h"
 #include "sbf_internal.h"
 #include "sbf_tile.cuh"
@@ -42,6 +43,73 @@ __device__ __forceinline__ void log_put(const RunLog& log, uint64_t at, uint32_t
     log.shards[at] = shard;
     *reinterpret_cast<ulonglong2*>(log.masks + 4 * at) = make_ulonglong2(m[0], m[1]);
     *reinterpret_cast<ulonglong2*>(log.masks + 4 * at + 2) = make_ulonglong2(m[2], m[3]);
+}
+
+// Insert: the mask of window j is T_j = OR of the one-hot masks of its F
+// s-mers; a super-k-mer run (consecutive valid windows with equal shard)
+// accumulates acc = OR T_j and is handed to flush(end, shard, acc) with end
+// non-zero when the next window leaves the run.  With four s-mers per window,
+// flush is called on every window with `end` as its predicate.
+template <class C, class Flush>
+__device__ __forceinline__ void insert_strip(const uint32_t* c, uint32_t vmask,
+                                             uint32_t shard_mask, const uint64_t* onehot,
+                                             Flush&& flush) {
+    constexpr int F = C::F;
+    uint64_t acc[4] = {0, 0, 0, 0};
+    uint32_t prev_shard = 0;
+    bool prev_valid = false;
+    if constexpr (F == 4) {
+        // T_j = P_j | P_{j+2} with pair masks P_x = m_x | m_{x+1}.
+        uint64_t m0[4], m1[4], m2[4];
+        smer_masks<C>(c, 0, m0, onehot);
+        smer_masks<C>(c, 1, m1, onehot);
+        smer_masks<C>(c, 2, m2, onehot);
+        uint64_t pa[4], pb[4];
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            pa[w] = m0[w] | m1[w];
+            pb[w] = m1[w] | m2[w];
+        }
+        for_each_shard<C>(c, shard_mask, [&](int j, uint32_t shard) {
+            uint64_t m3[4];
+            smer_masks<C>(c, j + 3, m3, onehot);
+            const bool valid = (vmask >> j) & 1u;
+            const bool cont = valid && prev_valid && shard == prev_shard;
+            flush((prev_valid && !cont) ? 1u : 0u, prev_shard, acc);
+            const uint64_t keep = cont ? ~uint64_t{0} : uint64_t{0};
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+                const uint64_t pc = m2[w] | m3[w];
+                acc[w] = (acc[w] & keep) | pa[w] | pc;
+                pa[w] = pb[w];
+                pb[w] = pc;
+                m2[w] = m3[w];
+            }
+            prev_shard = shard;
+            prev_valid = valid;
+        });
+    } else {
+        uint64_t mring[F][4];
+#pragma unroll
+        for (int o = 0; o < F - 1; ++o) smer_masks<C>(c, o, mring[o], onehot);
+        for_each_shard<C>(c, shard_mask, [&](int j, uint32_t shard) {
+            smer_masks<C>(c, j + F - 1, mring[(j + F - 1) % F], onehot);
+            const bool valid = (vmask >> j) & 1u;
+            const bool cont = valid && prev_valid && shard == prev_shard;
+            if (prev_valid && !cont) flush(1u, prev_shard, acc);
+            const uint64_t keep = cont ? ~uint64_t{0} : uint64_t{0};
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+                uint64_t t = mring[j % F][w];
+#pragma unroll
+                for (int o = 1; o < F; ++o) t |= mring[(j + o) % F][w];
+                acc[w] = (acc[w] & keep) | t;
+            }
+            prev_shard = shard;
+            prev_valid = valid;
+        });
+    }
+    if (prev_valid) flush(1u, prev_shard, acc);
 }
 
 // The insert tile path (plain loads for staging) with each super-k-mer run

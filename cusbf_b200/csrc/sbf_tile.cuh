@@ -23,23 +23,23 @@
 //     Gil-Werman sliding minimum over blocks of W positions (about 3
 //     comparisons per window, one more for W > 16, where the reference hashes
 //     and compares all W m-mers of every window).
-//   * Insert merges consecutive windows that select the same shard (a
-//     super-k-mer run) in registers and flushes each run with one 32-byte
-//     bulk OR-reduction (cp.reduce.async.bulk .or.b64) from a per-thread
-//     shared-memory ring: one L2 sector operation per run.
-//   * Query lists each strip's runs, gives the runs that hold a valid window
-//     consecutive slots of a per-warp shared-memory pool, and has the warp
-//     copy their 32-byte shards there with cp.async, a lane pair per shard
-//     (one request each).  It then tests the findere rule (all k-s+1 s-mers
-//     present) per window with byte permutes of the current run's shard.
-//   * Insert word masks come from a shared one-hot table (1 << b).
+//   * Both list a strip's super-k-mer runs (consecutive windows that select
+//     one shard) and give the runs that hold a valid window consecutive slots
+//     of a per-warp shared-memory pool; a run that crosses into the next
+//     strip is one run.
+//   * Query has the warp copy the runs' 32-byte shards to their slots with
+//     cp.async, a lane pair per shard (one request each), and tests the
+//     findere rule (all k-s+1 s-mers present) per window with byte permutes
+//     of the current run's shard.
+//   * Insert ORs the one-hot masks of a run's s-mers in registers, stores them
+//     to the run's slot, and has the warp OR the slots into their shards, four
+//     lanes and one request each.
 //   * Ragged launches take tiles from a device work-queue counter and drop
 //     windows that cross a record boundary or touch a byte outside every
 //     record (marked per tile in shared memory).
 #pragma once
 
 #include "sbf_device.cuh"
-#include "sbf_flush.cuh"
 #include "sbf_internal.h"
 
 namespace sbf {
@@ -303,17 +303,20 @@ __device__ __forceinline__ uint32_t strip_valid(uint64_t bits, int64_t first_kme
     return vmask;
 }
 
-// One-hot word masks of the s-mer at strip position r.  With four hashes
-// each word gets one bit, read from `onehot` (1 << b for b = 0..63 in the
-// CTA's shared memory): four table loads replace four 64-bit variable
-// shifts on the ALU pipe.
+// One-hot word masks of the s-mer at strip position r.  With four hashes each
+// word gets one bit: the first word's mask is read from `onehot` (1 << b for
+// b = 0..63 in the CTA's shared memory) and the others are 64-bit shifts.
+// The table spares the logic pipe two instructions a word, but 32 random
+// entries take about six passes of the shared-memory pipe: 100 Mbp took 531
+// us with four loads, 494 with three or two, 488 with one and 494 with none.
 template <class C>
 __device__ __forceinline__ void smer_masks(const uint32_t* c, int r, uint64_t m[4],
                                            const uint64_t* onehot) {
     const uint64_t h = smer_hash(smer_at<C>(c, r));
     if constexpr (C::H == 4) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) m[j] = onehot[bit_address<4>(h, j)];
+        for (int j = 0; j < 4; ++j)
+            m[j] = j == 0 ? onehot[bit_address<4>(h, j)] : uint64_t{1} << bit_address<4>(h, j);
     } else {
         m[0] = m[1] = m[2] = m[3] = 0;
 #pragma unroll
@@ -325,75 +328,6 @@ __device__ __forceinline__ void smer_masks(const uint32_t* c, int r, uint64_t m[
 // barrier publishes it).
 __device__ __forceinline__ void onehot_init(uint64_t* onehot) {
     if (threadIdx.x < 64) onehot[threadIdx.x] = uint64_t{1} << threadIdx.x;
-}
-
-// Insert: the mask of window j is T_j = OR of the one-hot masks of its F
-// s-mers; a super-k-mer run (consecutive valid windows with equal shard)
-// accumulates acc = OR T_j and is handed to flush(end, shard, acc) with end
-// non-zero when the next window leaves the run (the insert kernel ORs it
-// into the shard; the sharded insert's emit kernel records it).  With four
-// s-mers per window, flush is called on every window with `end` as its
-// predicate, so the per-run work needs no branch.
-template <class C, class Flush>
-__device__ __forceinline__ void insert_strip(const uint32_t* c, uint32_t vmask,
-                                             uint32_t shard_mask, const uint64_t* onehot,
-                                             Flush&& flush) {
-    constexpr int F = C::F;
-    uint64_t acc[4] = {0, 0, 0, 0};
-    uint32_t prev_shard = 0;
-    bool prev_valid = false;
-    if constexpr (F == 4) {
-        // T_j = P_j | P_{j+2} with pair masks P_x = m_x | m_{x+1}.
-        uint64_t m0[4], m1[4], m2[4];
-        smer_masks<C>(c, 0, m0, onehot);
-        smer_masks<C>(c, 1, m1, onehot);
-        smer_masks<C>(c, 2, m2, onehot);
-        uint64_t pa[4], pb[4];
-#pragma unroll
-        for (int w = 0; w < 4; ++w) {
-            pa[w] = m0[w] | m1[w];
-            pb[w] = m1[w] | m2[w];
-        }
-        for_each_shard<C>(c, shard_mask, [&](int j, uint32_t shard) {
-            uint64_t m3[4];
-            smer_masks<C>(c, j + 3, m3, onehot);
-            const bool valid = (vmask >> j) & 1u;
-            const bool cont = valid && prev_valid && shard == prev_shard;
-            flush((prev_valid && !cont) ? 1u : 0u, prev_shard, acc);
-            const uint64_t keep = cont ? ~uint64_t{0} : uint64_t{0};
-#pragma unroll
-            for (int w = 0; w < 4; ++w) {
-                const uint64_t pc = m2[w] | m3[w];
-                acc[w] = (acc[w] & keep) | pa[w] | pc;
-                pa[w] = pb[w];
-                pb[w] = pc;
-                m2[w] = m3[w];
-            }
-            prev_shard = shard;
-            prev_valid = valid;
-        });
-    } else {
-        uint64_t mring[F][4];
-#pragma unroll
-        for (int o = 0; o < F - 1; ++o) smer_masks<C>(c, o, mring[o], onehot);
-        for_each_shard<C>(c, shard_mask, [&](int j, uint32_t shard) {
-            smer_masks<C>(c, j + F - 1, mring[(j + F - 1) % F], onehot);
-            const bool valid = (vmask >> j) & 1u;
-            const bool cont = valid && prev_valid && shard == prev_shard;
-            if (prev_valid && !cont) flush(1u, prev_shard, acc);
-            const uint64_t keep = cont ? ~uint64_t{0} : uint64_t{0};
-#pragma unroll
-            for (int w = 0; w < 4; ++w) {
-                uint64_t t = mring[j % F][w];
-#pragma unroll
-                for (int o = 1; o < F; ++o) t |= mring[(j + o) % F][w];
-                acc[w] = (acc[w] & keep) | t;
-            }
-            prev_shard = shard;
-            prev_valid = valid;
-        });
-    }
-    if (prev_valid) flush(1u, prev_shard, acc);
 }
 
 __device__ __forceinline__ void cp_async_commit() {
@@ -841,6 +775,207 @@ __device__ __forceinline__ uint32_t query_strip_direct(uint32_t code_mem, uint32
 }
 
 // ---------------------------------------------------------------------------
+// Insert of one strip
+// ---------------------------------------------------------------------------
+
+// acc = a | b | c when `pred` is non-zero.
+__device__ __forceinline__ void or3_if(uint32_t pred, uint32_t (&acc)[8], const uint32_t (&a)[8],
+                                       const uint32_t (&b)[8], const uint32_t (&c)[8]) {
+#pragma unroll
+    for (int q = 0; q < 8; q += 4)
+        asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %16, 0;\n\t"
+            "@p lop3.b32 %0, %4, %8, %12, 0xFE;\n\t@p lop3.b32 %1, %5, %9, %13, 0xFE;\n\t"
+            "@p lop3.b32 %2, %6, %10, %14, 0xFE;\n\t@p lop3.b32 %3, %7, %11, %15, 0xFE;\n\t}"
+            : "+r"(acc[q]), "+r"(acc[q + 1]), "+r"(acc[q + 2]), "+r"(acc[q + 3])
+            : "r"(a[q]), "r"(a[q + 1]), "r"(a[q + 2]), "r"(a[q + 3]), "r"(b[q]), "r"(b[q + 1]),
+              "r"(b[q + 2]), "r"(b[q + 3]), "r"(c[q]), "r"(c[q + 1]), "r"(c[q + 2]),
+              "r"(c[q + 3]), "r"(pred));
+}
+
+// Stores a run's masks at shared address `at` and moves on to the next slot
+// (`at` becomes `next`) when `pred` is non-zero.
+__device__ __forceinline__ void store_run_if(uint32_t pred, uint32_t& at, uint32_t& next,
+                                             const uint32_t (&acc)[8]) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t"
+        "@p st.shared.v4.u32 [%0], {%3, %4, %5, %6};\n\t"
+        "@p st.shared.v4.u32 [%0+16], {%7, %8, %9, %10};\n\t"
+        "@p mov.u32 %0, %1;\n\t@p add.u32 %1, %1, 32;\n\t}"
+        : "+r"(at), "+r"(next)
+        : "r"(pred), "r"(acc[0]), "r"(acc[1]), "r"(acc[2]), "r"(acc[3]), "r"(acc[4]), "r"(acc[5]),
+          "r"(acc[6]), "r"(acc[7])
+        : "memory");
+}
+
+// *dst |= *src, 32 bytes of shared memory.
+__device__ __forceinline__ void or_slot(uint32_t dst, uint32_t src) {
+#pragma unroll
+    for (int q = 0; q < 32; q += 16)
+        asm volatile(
+            "{\n\t.reg .b32 a<4>, b<4>;\n\t"
+            "ld.shared.v4.u32 {a0, a1, a2, a3}, [%0];\n\t"
+            "ld.shared.v4.u32 {b0, b1, b2, b3}, [%1];\n\t"
+            "or.b32 a0, a0, b0;\n\tor.b32 a1, a1, b1;\n\t"
+            "or.b32 a2, a2, b2;\n\tor.b32 a3, a3, b3;\n\t"
+            "st.shared.v4.u32 [%0], {a0, a1, a2, a3};\n\t}" ::"r"(dst + q),
+            "r"(src + q)
+            : "memory");
+}
+
+// ORs the slots below `total` into their shards, four lanes a slot with one
+// 8-byte reduction each: the four make one 32-byte request.  (One 32-byte
+// bulk reduction per slot takes 72 G slots/s from an L2-resident filter where
+// this takes 120, and both 20 to 31 G/s from larger ones.  It also holds the
+// slot until it is read.)
+__device__ __forceinline__ void flush_slots(uint32_t total, uint32_t pool, uint32_t ids,
+                                            uint32_t shard_mask, uint64_t* words) {
+    const uint32_t lane = threadIdx.x & 31;
+    uint64_t* word = words + (lane & 3u);
+    uint32_t id = ids + 4 * (lane >> 2), src = pool + 8 * lane;
+    for (uint32_t e = lane >> 2; __any_sync(0xFFFFFFFFu, e < total); e += 32) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t.reg .b32 s;\n\t.reg .b64 a, v;\n\t"
+                "setp.lt.u32 p, %0, %1;\n\t"
+                "@p ld.shared.u32 s, [%2];\n\t"
+                "@p ld.shared.u64 v, [%5];\n\t"
+                "@p and.b32 s, s, %3;\n\t"
+                "@p mad.wide.u32 a, s, 32, %4;\n\t"
+                "@p red.relaxed.gpu.global.or.b64 [a], v;\n\t}" ::"r"(e + 8 * u),
+                "r"(total), "r"(id + 32 * u), "r"(shard_mask), "l"(word), "r"(src + 256 * u)
+                : "memory");
+        id += 128;
+        src += 1024;
+    }
+}
+
+// Insert of one strip.  The minimizer pass lists the strip's runs as in a
+// query.  The mask pass then walks the windows: the mask of a run is the OR of
+// the one-hot masks of all its windows' s-mers, kept in registers and stored
+// to a pool slot at the run's last window.  A first run that continues the
+// left lane's last one is ORed into that lane's slot.  At the end the warp
+// flushes the slots.
+//
+// Bound: the memory's rate of random read-modify-writes for filters beyond L2
+// (20 G shards/s at 8 GiB, 31 at 256 MiB), else the integer logic pipe.  3.1
+// Gbp into 8 GiB 18.4 ms and 100 Mbp into 256 MiB 488 us; with each window
+// issuing the flush of a run that ends there (a predicated 32-byte bulk
+// reduction, strips flushing the runs between them twice) it was 21.1 ms and
+// 688 us.
+template <class C>
+__device__ __forceinline__ void insert_strip_runs(uint32_t code_mem, uint32_t vmask,
+                                                  uint32_t shard_mask, uint64_t* words,
+                                                  uint32_t run_mem, const uint64_t* onehot) {
+    constexpr int F = C::F;
+    constexpr uint32_t kPoolSlots = insert_pool_slots(C::W, C::H);
+    static_assert(kPoolSlots * 32 >= 32 * 128, "the run lists fit the pool");
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t ids = run_mem + 32 * kPoolSlots;
+    const uint32_t spare = ids + 4 * kPoolSlots + 32 * lane;
+    while (__any_sync(0xFFFFFFFFu, vmask != 0u)) {
+        const uint32_t list = run_mem + 4 * lane;
+        const uint3 runs = list_runs<C>(code_mem, list);
+        const uint32_t chg = runs.x;
+        uint32_t heads = vmask & (chg | ~(vmask << 1));
+        const int n = __popc(heads);
+        const bool lend = n > 0 && (vmask >> (kStrip - 1)) && !(n == 1 && (vmask & 1u));
+        const uint32_t left_lo = __shfl_up_sync(0xFFFFFFFFu, runs.z, 1);
+        const uint32_t lenders = __ballot_sync(0xFFFFFFFFu, lend);
+        bool merge =
+            lane > 0 && (heads & 1u) && (lenders >> (lane - 1) & 1u) && left_lo == runs.y;
+        const uint32_t own = n - (merge ? 1 : 0);
+        uint32_t end = own;
+#pragma unroll
+        for (int o = 1; o < 32; o *= 2) {
+            const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, end, o);
+            if (lane >= static_cast<uint32_t>(o)) end += v;
+        }
+        const uint32_t begin = end - own;
+        const bool fits = end <= kPoolSlots;
+        // Windows that end a run: the next one is invalid or a head.
+        uint32_t ends = vmask & ~((vmask & ~heads) >> 1);
+        if (!fits) {
+            heads = ends = 0;
+            merge = false;
+        }
+        uint32_t rest = merge ? heads & (heads - 1u) : heads;
+        for (uint32_t at = ids + 4 * begin; __any_sync(0xFFFFFFFFu, rest != 0u); at += 4) {
+            const uint32_t b = rest & (0u - rest);
+            rest ^= b;
+            const uint32_t e = __popc(chg & (b ^ (b - 1u))) - 1;
+            copy_u32_if(b, at, list + 128 * e);
+        }
+        __syncwarp();
+        uint32_t c[kStripWords];
+        load_code_words(code_mem, c);
+        uint32_t ring[F][8];
+        auto enter = [&](int r) {
+            uint64_t m[4];
+            smer_masks<C>(c, r, m, onehot);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                ring[r % F][2 * q] = static_cast<uint32_t>(m[q]);
+                ring[r % F][2 * q + 1] = static_cast<uint32_t>(m[q] >> 32);
+            }
+        };
+#pragma unroll
+        for (int o = 0; o < F - 1; ++o) enter(o);
+        uint32_t acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        uint32_t at = merge ? spare : run_mem + 32 * begin;
+        uint32_t next = run_mem + 32 * (merge ? begin : begin + 1);
+#pragma unroll 1
+        for (int turn = 0; turn < 2; ++turn) {
+#pragma unroll
+            for (int j = 0; j < kTurn; ++j) {
+                enter(j + F - 1);
+                const uint32_t head = heads & (1u << j);
+                if constexpr (F == 4) {
+                    or3_if(head, acc, ring[j % F], ring[(j + 1) % F], ring[(j + 2) % F]);
+                } else {
+                    const uint32_t keep = head ? 0u : 0xFFFFFFFFu;
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        uint32_t u = acc[q] & keep;
+#pragma unroll
+                        for (int o = 0; o < F - 1; ++o) u |= ring[(j + o) % F][q];
+                        acc[q] = u;
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < 8; ++q) acc[q] |= ring[(j + F - 1) % F][q];
+                store_run_if(ends & (1u << j), at, next, acc);
+            }
+            heads >>= kTurn;
+            ends >>= kTurn;
+            c[0] = c[1];
+            c[1] = c[2];
+            c[2] = c[3];
+            if constexpr (kTurn % F != 0) {
+                uint32_t old[F][8];
+#pragma unroll
+                for (int i = 0; i < F; ++i) {
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) old[i][q] = ring[i][q];
+                }
+#pragma unroll
+                for (int i = 0; i < F; ++i) {
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) ring[i][q] = old[(i + kTurn) % F][q];
+                }
+            }
+        }
+        __syncwarp();
+        if (merge) or_slot(run_mem + 32 * (begin - 1), spare);
+        __syncwarp();
+        flush_slots(__reduce_max_sync(0xFFFFFFFFu, fits ? end : 0u), run_mem, ids, shard_mask,
+                    words);
+        __syncwarp();  // the slots are read before another round's lists replace them
+        if (fits) vmask = 0;
+    }
+}
+
+// ---------------------------------------------------------------------------
 // The tile kernel
 // ---------------------------------------------------------------------------
 
@@ -974,7 +1109,10 @@ __device__ __forceinline__ void tally_records(const TileParams& p, uint32_t firs
 // Either way tile i+2 is taken while tile i is processed, and tile i+1's
 // staging copy is issued once tile i's bytes are encoded, into the same buffer.
 template <class C, bool kQuery, bool kDense, bool kRagged>
-__global__ void __launch_bounds__(kThreads, kQuery && query_three_ctas(C::W, C::H) ? 3 : 2)
+__global__ void __launch_bounds__(kThreads, (kQuery ? query_three_ctas(C::W, C::H)
+                                                    : insert_three_ctas(C::W, C::H))
+                                                ? 3
+                                                : 2)
     tile_kernel(TileParams p) {
     __shared__ alignas(128) uint8_t stage[kStageBytes];
     __shared__ alignas(8) uint32_t code[kCodeWords + 4];
@@ -1023,8 +1161,6 @@ __global__ void __launch_bounds__(kThreads, kQuery && query_three_ctas(C::W, C::
     // warp (query_cta_bytes per CTA), or the insert kernel's flush staging ring,
     // [slot][thread] (kInsertSlotBytes per CTA).
     extern __shared__ __align__(16) uint64_t slots[];
-    FlushRing ring{slots + 4 * tid, 0u};
-    (void)ring;
     unsigned long long n_valid = 0, n_pos = 0;
     const uint32_t origin = stage_origin<kDense>(p);
     for (uint32_t it = 0;; ++it) {
@@ -1040,7 +1176,6 @@ __global__ void __launch_bounds__(kThreads, kQuery && query_three_ctas(C::W, C::
                 (void)mbar_wait_bounded(&bar, it & 1u);
             }
             __syncthreads();
-            if constexpr (!kQuery) flush_ring_drain();
             return;
         }
         if (!covered) {
@@ -1069,9 +1204,6 @@ __global__ void __launch_bounds__(kThreads, kQuery && query_three_ctas(C::W, C::
             take(it + 2, (it + 2) % 3);
         }
 
-        uint32_t c[kStripWords];
-#pragma unroll
-        for (int q = 0; q < kStripWords; ++q) c[q] = code[tid * (kStrip / 16) + q];
         static_assert(kStrip == 32 && kStripWords == 4, "a strip's bits are two 32-bit words");
         auto strip_bits = [&](const uint32_t* a) {
             return static_cast<uint64_t>(a[tid]) | (static_cast<uint64_t>(a[tid + 1]) << 32);
@@ -1083,8 +1215,8 @@ __global__ void __launch_bounds__(kThreads, kQuery && query_three_ctas(C::W, C::
             n_valid += __popc(vmask);
         }
         uint32_t hits = 0;
+        const uint32_t code_mem = smem_addr(code + tid * (kStrip / 16));
         if constexpr (kQuery) {
-            const uint32_t code_mem = smem_addr(code + tid * (kStrip / 16));
             if constexpr (C::W < 6 && C::M <= 8) {
                 hits = query_strip_direct<C>(code_mem, vmask, p.shard_mask, p.words);
             } else {
@@ -1099,17 +1231,14 @@ __global__ void __launch_bounds__(kThreads, kQuery && query_three_ctas(C::W, C::
             if (p.out_bits && first_kmer < static_cast<int64_t>(p.n_kmers))
                 p.out_bits[first_kmer >> 5] = hits;
         } else {
-            if (vmask)
-                insert_strip<C>(c, vmask, p.shard_mask, onehot,
-                                [&](uint32_t end, uint32_t shard, const uint64_t* acc) {
-                                    flush_run_if(end, p.words, shard, acc, ring);
-                                });
+            constexpr int kWarpBytes = insert_warp_bytes(C::W, C::H);
+            insert_strip_runs<C>(code_mem, vmask, p.shard_mask, p.words,
+                                 smem_addr(slots) + (tid >> 5) * kWarpBytes, onehot);
         }
         if constexpr (kRagged) {
             if (p.rec_valid) tally_records(p, first_rec[it % 3], first_kmer, vmask, hits);
         }
     }
-    if constexpr (!kQuery) flush_ring_drain();
     if constexpr (kRagged) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {

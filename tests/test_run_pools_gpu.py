@@ -1,0 +1,88 @@
+"""The tile kernels' run lists and slot pools against the oracle, where a pool
+takes one round, several rounds or none, and at the edges of strips (32
+windows), warps (1024) and tiles (8192)."""
+import numpy as np
+import pytest
+
+from conftest import random_dna
+
+pytestmark = pytest.mark.gpu
+
+CONFIGS = [
+    dict(k=31, s=28, m=16, hashes=4),   # W = 16, F = 4
+    dict(k=21, s=19, m=11, hashes=4),   # W = 11, F = 3
+    dict(k=31, s=28, m=16, hashes=8),
+    dict(k=31, s=28, m=16, hashes=16),
+    dict(k=31, s=30, m=21, hashes=4),   # F = 2
+    dict(k=31, s=26, m=28, hashes=4),   # W = 4: several rounds, F = 6
+    dict(k=31, s=28, m=31, hashes=4),   # W = 1: every window a run
+    dict(k=28, s=26, m=6, hashes=12),   # W = 23
+    dict(k=5, s=4, m=3, hashes=4),      # W = 3, few m-mers: no pool
+]
+
+
+LENGTHS = (1, 31, 32, 33, 1023, 1024, 1025, 8191, 8192, 8193, 1 << 20)
+IDS = ["-".join(map(str, c.values())) for c in CONFIGS]
+
+
+def sequences(k, m):
+    """A genome with a short period, a homopolymer and a run of N, and a mixed
+    sequence that shares parts of it and has invalid bases at every spacing up
+    to twice the window length."""
+    rng = np.random.default_rng(k * 100 + m)
+    genome = random_dna(rng, 60_000)
+    genome[20_000:21_000] = np.resize(random_dna(rng, 7), 1_000)
+    genome[30_000:30_500] = ord("A")
+    genome[40_000:40_400] = ord("N")
+    gaps = random_dna(rng, 20_000)
+    at, step = 0, 1
+    while at < gaps.size:
+        gaps[at] = ord("N")
+        at += step
+        step = step % (2 * k) + 1
+    return genome, np.concatenate([genome[10_000:45_000], random_dna(rng, 20_000), gaps,
+                                   genome[:5_000]])
+
+
+def on_device(torch, seq, shift):
+    d = torch.zeros(seq.size + 16, dtype=torch.uint8, device="cuda")[shift:][:seq.size]
+    return d.copy_(torch.from_numpy(seq.copy()))
+
+
+@pytest.mark.parametrize("cfg", CONFIGS, ids=IDS)
+def test_insert_matches_oracle(sbf, cuda, oracle_mod, cfg):
+    _, mixed = sequences(cfg["k"], cfg["m"])
+    o = oracle_mod.Oracle(**cfg)
+    f = sbf.Filter(1 << 18, **cfg)
+    for n in LENGTHS:
+        for shift in (0, 3):
+            seq = mixed[shift:][:n + cfg["k"] - 1]
+            words = o.new_words(1 << 18)
+            o.insert(words, seq)
+            f.clear()
+            f.insert_sequence_async(on_device(cuda, seq, shift))
+            np.testing.assert_array_equal(f.words_host(), words)
+
+
+@pytest.mark.parametrize("cfg", CONFIGS, ids=IDS)
+def test_query_matches_oracle(sbf, cuda, oracle_mod, cfg):
+    torch = cuda
+    k = cfg["k"]
+    genome, mixed = sequences(k, cfg["m"])
+    o = oracle_mod.Oracle(**cfg)
+    words = o.new_words(1 << 18)
+    o.insert(words, genome)
+    f = sbf.Filter(1 << 18, **cfg)
+    f.insert_sequence_async(torch.from_numpy(genome).cuda())
+    for n in LENGTHS:
+        for shift in (0, 3):
+            seq = mixed[shift:][:n + k - 1]
+            want = o.contains(words, seq)
+            d = on_device(torch, seq, shift)
+            out = torch.full((want.size,), 7, dtype=torch.uint8, device="cuda")
+            f.contains_sequence_async(d, out)
+            bits = torch.full(((want.size + 31) // 32,), -1, dtype=torch.int32, device="cuda")
+            f.contains_sequence_bits_async(d, bits)
+            np.testing.assert_array_equal(out.cpu().numpy(), want)
+            got = np.unpackbits(bits.cpu().numpy().view(np.uint8), bitorder="little")
+            np.testing.assert_array_equal(got[:want.size], want)
