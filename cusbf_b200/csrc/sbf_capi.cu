@@ -172,17 +172,15 @@ int sbf_filter::launch(bool query, bool dense, const void* input, uint64_t input
     p.shard_mask = static_cast<uint32_t>(num_shards - 1);
     p.out = out_bits ? nullptr : out;
     p.out_bits = out_bits;
-    p.n_tiles = (n_kmers + static_cast<uint64_t>(phase) + kTileKmers - 1) / kTileKmers;
+    const int which = (query ? 1 : 0) + (dense ? 2 : 0);
+    const StripKernel kernel = strip_kernel(ks, which, n_kmers, device, sms);
+    const uint64_t tile = kernel.tile_kmers();
+    p.n_tiles = (n_kmers + static_cast<uint64_t>(phase) + tile - 1) / tile;
     p.err = d_err;
     p.gen = gen;
-    const int which = (query ? 1 : 0) + (dense ? 2 : 0);
-    const void* fn = which == 0   ? ks->insert_bytes
-                     : which == 1 ? ks->query_bytes
-                     : which == 2 ? ks->insert_dense
-                                  : ks->query_dense;
     const uint64_t resident = static_cast<uint64_t>(sms) * static_cast<uint64_t>(occupancy[which]);
     const uint64_t grid = std::min<uint64_t>(p.n_tiles, std::max<uint64_t>(resident, 1));
-    SBF_CUDA(launch_set_kernel(ks, fn, static_cast<unsigned>(grid), query, p, st));
+    SBF_CUDA(launch_set_kernel(ks, kernel.fn, static_cast<unsigned>(grid), query, p, st));
     ++launches;
     return SBF_OK;
 }

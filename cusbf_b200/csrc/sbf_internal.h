@@ -13,7 +13,7 @@ namespace sbf {
 constexpr int kThreads = 256;                          // threads per CTA
 constexpr int kStrip = 32;                             // consecutive k-mers per thread
 constexpr int kTileKmers = kThreads * kStrip;          // k-mers per tile (8192)
-constexpr int kStripWords = kStrip / 16 + 2;           // code words one strip reads
+constexpr int kStripWords = 4;                         // code words one strip reads
 constexpr int kCodeWords = (kThreads - 1) * (kStrip / 16) + kStripWords;  // per tile
 constexpr int kStageBytes = kCodeWords * 16 + 64;      // staged input bytes per buffer
 constexpr int kFlushSlots = 8;                         // insert bulk-reduce staging slots
@@ -134,8 +134,26 @@ struct KernelSet {
     int smem_query = query_cta_bytes(k - m + 1, h);
     bool jit = false;    // loaded from a run-time compiled library
     int jit_occupancy = 2;  // resident CTAs per SM assumed for run-time compiled sets
+    const void* fn(int which) const {
+        const void* const fns[6] = {insert_bytes, query_bytes,   insert_dense,
+                                    query_dense,  insert_ragged, query_ragged};
+        return fns[which];
+    }
     int smem(bool query) const { return query ? smem_query : smem_insert; }
 };
+
+// Which of a set's kernels: insert or query of bytes, dense words, records.
+enum { kInsertBytes, kQueryBytes, kInsertDense, kQueryDense, kInsertRagged, kQueryRagged };
+
+// A kernel and the windows per thread it was compiled for.
+struct StripKernel {
+    const void* fn;
+    int strip;
+    uint64_t tile_kmers() const { return static_cast<uint64_t>(kThreads) * strip; }
+};
+// The kernel of a launch of `n_kmers` windows: a set's own, or one with
+// narrower strips when the launch is small.
+StripKernel strip_kernel(const KernelSet* ks, int which, uint64_t n_kmers, int device, int sms);
 
 // Returns the kernel table for a configuration, or nullptr when it is not
 // compiled into this library.
@@ -149,7 +167,8 @@ cudaError_t launch_pack_dense(const uint8_t* seq, uint64_t num_symbols, uint64_t
 // Ragged launches: tile_rec[t] = first record whose end exceeds the first
 // input byte of tile t (n_ranges when none).
 cudaError_t launch_tile_records(const DevRange* ranges, uint64_t n_ranges, int64_t sym_base,
-                                uint64_t n_tiles, uint32_t* tile_rec, cudaStream_t stream);
+                                uint64_t tile_kmers, uint64_t n_tiles, uint32_t* tile_rec,
+                                cudaStream_t stream);
 // The same with the record and tile counts read from `sizes` on the device;
 // `max_tiles` bounds the launch.
 cudaError_t launch_tile_records_sized(const DevRange* ranges, const DevSizes* sizes,

@@ -3,8 +3,10 @@
 // run time by sbf_jit.cpp) and the auxiliary kernels.
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 
+#include "sbf_configs.h"
 #include "sbf_device.cuh"
 #include "sbf_internal.h"
 #include "sbf_tile.cuh"
@@ -14,10 +16,10 @@ namespace sbf {
 // tile_rec[t] = first record whose end exceeds the first byte tile t stages
 // (binary search; records sorted and non-overlapping).
 __global__ void tile_records_kernel(const DevRange* ranges, uint64_t n, int64_t sym_base,
-                                    uint64_t n_tiles, uint32_t* tile_rec) {
+                                    uint64_t tile_kmers, uint64_t n_tiles, uint32_t* tile_rec) {
     const uint64_t t = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= n_tiles) return;
-    const int64_t s0 = static_cast<int64_t>(t) * kTileKmers + sym_base;
+    const int64_t s0 = static_cast<int64_t>(t * tile_kmers) + sym_base;
     uint64_t lo = 0, hi = n;
     while (lo < hi) {
         const uint64_t mid = (lo + hi) >> 1;
@@ -93,10 +95,11 @@ cudaError_t launch_pack_dense(const uint8_t* seq, uint64_t num_symbols, uint64_t
 const void* tile_records_kernel_ptr() { return reinterpret_cast<const void*>(&tile_records_kernel); }
 
 cudaError_t launch_tile_records(const DevRange* ranges, uint64_t n_ranges, int64_t sym_base,
-                                uint64_t n_tiles, uint32_t* tile_rec, cudaStream_t stream) {
+                                uint64_t tile_kmers, uint64_t n_tiles, uint32_t* tile_rec,
+                                cudaStream_t stream) {
     if (n_tiles == 0) return cudaSuccess;
     tile_records_kernel<<<static_cast<unsigned>((n_tiles + 255) / 256), 256, 0, stream>>>(
-        ranges, n_ranges, sym_base, n_tiles, tile_rec);
+        ranges, n_ranges, sym_base, tile_kmers, n_tiles, tile_rec);
     return cudaGetLastError();
 }
 
@@ -145,18 +148,55 @@ KernelSet make_set() {
 }
 
 static const KernelSet kSets[] = {
-    make_set<31, 28, 16, 4>(),  // the benchmark configuration
-    make_set<31, 30, 16, 4>(),  make_set<31, 31, 16, 4>(), make_set<31, 28, 16, 8>(),
-    make_set<31, 28, 16, 16>(), make_set<21, 19, 11, 4>(), make_set<5, 4, 3, 4>(),
-    make_set<3, 2, 2, 4>(),
-    // The reference's FPR sweep over s (benchmarks/fpr_fastx_sweep.cu:294-302).
-    make_set<31, 28, 21, 4>(), make_set<31, 30, 21, 4>(), make_set<31, 31, 21, 4>(),
+#define SBF_SET(K, S, M, H) make_set<K, S, M, H>(),
+    SBF_COMPILED_CONFIGS(SBF_SET)
+#undef SBF_SET
 };
+constexpr int kNumSets = static_cast<int>(sizeof kSets / sizeof kSets[0]);
 
 const KernelSet* find_kernels(int k, int s, int m, int h) {
     for (const KernelSet& ks : kSets)
         if (ks.k == k && ks.s == s && ks.m == m && ks.h == h) return &ks;
     return nullptr;
+}
+
+// Windows per thread of a launch.  A strip's windows are worked off one after
+// the other, so a launch that gives every SM few warps takes as long as one
+// strip; shorter strips cost more work per window (W - 1 m-mers and F - 1
+// s-mers beyond its windows) but spread over more of the chip.  <31,28,16,4>
+// insert / query with strips of 8, 16 and 32 windows, in us:
+//    30 k windows   6.7 / 5.0    7.3 / 6.3   10.3 / 8.3
+//   400 k           8.3 / 6.3    8.3 / 6.3   10.3 / 8.6
+//   1.5 M          16.5 / 12.4  12.8 / 10.3  15.6 / 12.4
+//     3 M          26.4 / 20.6  22.6 / 18.5  20.6 / 16.5
+// so strips of 8 take up to two tiles an SM, strips of 16 up to three.
+static int narrow_strip(uint64_t n_kmers, int sms) {
+    const uint64_t per_sm = n_kmers / static_cast<uint64_t>(sms > 0 ? sms : 1);
+    return per_sm < 2 * 8 * kThreads ? 8 : per_sm < 3 * 16 * kThreads ? 16 : kStrip;
+}
+
+const void* narrow16_kernel(int config, int which);
+const void* narrow8_kernel(int config, int which);
+
+StripKernel strip_kernel(const KernelSet* ks, int which, uint64_t n_kmers, int device, int sms) {
+    const StripKernel own{ks->fn(which), kStrip};
+    const int strip = narrow_strip(n_kmers, sms);
+    int config = 0;
+    while (config < kNumSets && ks != &kSets[config]) ++config;
+    if (strip == kStrip || config == kNumSets || device < 0 || device >= 64) return own;
+    const void* fn = strip == 16 ? narrow16_kernel(config, which) : narrow8_kernel(config, which);
+    // Devices on which the kernel may use its dynamic shared memory.
+    static std::atomic<uint64_t> ready[kNumSets][2][6];
+    std::atomic<uint64_t>& devices = ready[config][strip == 16][which];
+    if (!(devices.load(std::memory_order_acquire) >> device & 1u)) {
+        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 ks->smem((which & 1) != 0)) != cudaSuccess) {
+            cudaGetLastError();
+            return own;
+        }
+        devices.fetch_or(uint64_t{1} << device, std::memory_order_release);
+    }
+    return {fn, strip};
 }
 
 cudaError_t launch_set_kernel(const KernelSet* ks, const void* fn, unsigned grid, bool query,

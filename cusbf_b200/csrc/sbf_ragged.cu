@@ -213,13 +213,13 @@ static unsigned ragged_grid(const sbf_filter* f, bool query, uint64_t n_tiles, u
 }
 
 int ragged_launch(sbf_filter* f, bool query, const TileParams& p, uint32_t ctas,
-                         cudaStream_t st) {
+                  cudaStream_t st, StripKernel kernel) {
     if (p.n_tiles == 0) return SBF_OK;
-    SBF_CUDA(launch_tile_records(p.ranges, p.n_ranges, p.sym_base, p.n_tiles,
+    if (!kernel.fn) kernel = {f->ks->fn(query ? kQueryRagged : kInsertRagged), kStrip};
+    SBF_CUDA(launch_tile_records(p.ranges, p.n_ranges, p.sym_base, kernel.tile_kmers(), p.n_tiles,
                                  const_cast<uint32_t*>(p.tile_rec), st));
     SBF_CUDA(cudaMemsetAsync(p.queue, 0, sizeof(unsigned int), st));
-    const void* fn = query ? f->ks->query_ragged : f->ks->insert_ragged;
-    SBF_CUDA(launch_set_kernel(f->ks, fn, ragged_grid(f, query, p.n_tiles, ctas), query, p, st));
+    SBF_CUDA(launch_set_kernel(f->ks, kernel.fn, ragged_grid(f, query, p.n_tiles, ctas), query, p, st));
     f->launches += 2;
     return SBF_OK;
 }
@@ -235,9 +235,10 @@ int ragged_graph_launch(sbf_filter* f, RaggedGraph& g, bool query, const TilePar
     const DevRange* a_rng = p.ranges;
     uint64_t a_n = p.n_ranges;
     int64_t a_base = p.sym_base;
+    uint64_t a_tile_kmers = kTileKmers;
     uint64_t a_tiles = p.n_tiles;
     uint32_t* a_rec = const_cast<uint32_t*>(p.tile_rec);
-    void* rec_args[] = {&a_rng, &a_n, &a_base, &a_tiles, &a_rec};
+    void* rec_args[] = {&a_rng, &a_n, &a_base, &a_tile_kmers, &a_tiles, &a_rec};
     TileParams tp = p;
     void* tile_args[] = {&tp};
     cudaKernelNodeParams rk{};
@@ -605,9 +606,13 @@ static int ragged_async(sbf_filter_t* f, bool query, const char* d_seq, uint64_t
                                           : ctl_counts(r));
     p.rec_valid = reinterpret_cast<unsigned long long*>(d_rec_valid);
     p.rec_pos = reinterpret_cast<unsigned long long*>(d_rec_pos);
+    const StripKernel kernel = strip_kernel(f->ks, query ? kQueryRagged : kInsertRagged, p.n_kmers,
+                                            f->device, f->sms);
+    const uint64_t tile = kernel.tile_kmers();
+    p.n_tiles = (p.n_kmers + static_cast<uint64_t>(-p.sym_base) + tile - 1) / tile;
     SBF_TRY(r->direct_tile_rec.ensure(p.n_tiles * 4 + 64));
     p.tile_rec = static_cast<const uint32_t*>(r->direct_tile_rec.ptr);
-    return ragged_launch(f, query, p, 0, st);
+    return ragged_launch(f, query, p, 0, st, kernel);
 }
 
 extern "C" int sbf_ragged_insert_async(sbf_filter_t* f, const char* d_seq, uint64_t len,

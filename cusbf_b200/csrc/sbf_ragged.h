@@ -19,9 +19,10 @@ TileParams ragged_params(const sbf_filter* f, bool query, const uint8_t* d_seq, 
                          uint8_t* d_out, unsigned int* queue, unsigned long long* counts,
                          bool out_bits = false);
 
-// Stream launch of one ragged pass: tile records, queue reset, tile kernel.
+// Stream launch of one ragged pass: tile records, queue reset, tile kernel (the
+// set's own unless `kernel` is given; p.n_tiles counts its tiles).
 int ragged_launch(sbf_filter* f, bool query, const TileParams& p, uint32_t ctas,
-                  cudaStream_t st);
+                  cudaStream_t st, StripKernel kernel = {nullptr, kStrip});
 
 // The same pass replayed as a graph whose two kernel nodes are updated per
 // launch (built on first use).

@@ -15,6 +15,7 @@
 #include <cstdint>
 
 #include "../../include/sbf_b200.h"
+#include "sbf_configs.h"
 #include "sbf_flush.cuh"
 #include "sbf_host.h"
 #include "sbf_internal.h"
@@ -132,7 +133,7 @@ __global__ void __launch_bounds__(kThreads, 2) emit_kernel(TileParams p, RunLog 
     onehot_init(onehot);  // published by the barrier at the top of the tile loop
     unsigned long long n_valid = 0;
     for (uint64_t tile = blockIdx.x; tile < p.n_tiles; tile += gridDim.x) {
-        TileGeom g = tile_geom<false>(p, tile);
+        TileGeom g = tile_geom<C, false>(p, tile);
         g.hi = g.lo;  // no bulk copy: every readable byte by plain loads
         __syncthreads();
         fill_ragged<false>(p, g, stage);
@@ -222,10 +223,9 @@ constexpr EmitSet emit_set() {
 
 // The configurations whose tile kernels are compiled into the library.
 const EmitSet kEmitSets[] = {
-    emit_set<31, 28, 16, 4>(),  emit_set<31, 30, 16, 4>(), emit_set<31, 31, 16, 4>(),
-    emit_set<31, 28, 16, 8>(),  emit_set<31, 28, 16, 16>(), emit_set<21, 19, 11, 4>(),
-    emit_set<5, 4, 3, 4>(),     emit_set<3, 2, 2, 4>(),     emit_set<31, 28, 21, 4>(),
-    emit_set<31, 30, 21, 4>(),  emit_set<31, 31, 21, 4>(),
+#define SBF_EMIT(K, S, M, H) emit_set<K, S, M, H>(),
+    SBF_COMPILED_CONFIGS(SBF_EMIT)
+#undef SBF_EMIT
 };
 
 const EmitSet* find_emit(const sbf_filter* f) {

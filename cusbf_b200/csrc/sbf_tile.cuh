@@ -8,8 +8,8 @@
 // and their dense-packed twins).  Results are bit-identical to it; the work
 // decomposition is new:
 //
-//   * A persistent CTA (two or three per SM) walks tiles of 8192 consecutive windows
-//     (kTileKmers).  Each tile's input bytes are staged into shared memory by
+//   * A persistent CTA (two or three per SM) walks tiles of 8192 consecutive
+//     windows (2048 or 4096 in small launches).  Each tile's input bytes are staged into shared memory by
 //     a 1D bulk async copy (TMA) on an mbarrier, issued as soon as the tile
 //     before it is encoded, so copies overlap hashing.  Only the 16-byte aligned
 //     interior goes through the bulk copy; ragged edges are read with plain
@@ -17,7 +17,8 @@
 //     is bounded and reports kDevErrStageTimeout instead of hanging.
 //   * Staged bytes are encoded with SWAR into 2-bit code words (16 bases per
 //     32-bit word, earliest base in the top bits) plus invalid masks.
-//   * Each of the 256 threads owns a strip of 32 consecutive windows.  Every
+//   * Each of the 256 threads owns a strip of 32 consecutive windows (8 or
+//     16 in small launches).  Every
 //     m-mer and s-mer of the strip is a funnel shift of the code words,
 //     every position is hashed once, and the per-window minimizer is a
 //     Gil-Werman sliding minimum over blocks of W positions (about 3
@@ -44,7 +45,8 @@
 
 namespace sbf {
 
-template <int K_, int S_, int M_, int H_>
+// A filter configuration and the windows per thread (strip).
+template <int K_, int S_, int M_, int H_, int Strip_ = kStrip>
 struct Cfg {
     static constexpr int K = K_;
     static constexpr int S = S_;
@@ -52,6 +54,15 @@ struct Cfg {
     static constexpr int H = H_;
     static constexpr int W = K - M + 1;  // m-mers per window
     static constexpr int F = K - S + 1;  // s-mers per window (findere span)
+    static constexpr int kStrip = Strip_;
+    static constexpr int kTileKmers = kThreads * kStrip;
+    static constexpr int kCodeWords = (kThreads - 1) * kStrip / 16 + kStripWords;
+    static constexpr int kStageBytes = kCodeWords * 16 + 64;
+    // The passes over a strip's windows take them in turns of at most 16.
+    static constexpr int kTurn = kStrip < 16 ? kStrip : 16;
+    static constexpr int kTurns = kStrip / kTurn;
+    static_assert(kStrip == 8 || kStrip == 16 || kStrip == 32, "strips of 8, 16 or 32 windows");
+    static_assert(kTileKmers / 4 % 16 == 0, "tiles start at one phase of 16 bytes");
     static_assert(K >= 1 && K <= 32, "k must fit a 64-bit packed window");
     static_assert(M >= 1 && M <= K, "m must satisfy 1 <= m <= k");
     static_assert(S >= 1 && S <= K, "s must satisfy 1 <= s <= k");
@@ -72,22 +83,23 @@ struct TileGeom {
     int64_t s0;      // symbol index of the tile's first grid position
 };
 
+template <class C>
 __device__ __forceinline__ int64_t tile_first_symbol(const TileParams& p, uint64_t tile) {
-    return static_cast<int64_t>(tile) * kTileKmers + p.sym_base;
+    return static_cast<int64_t>(tile) * C::kTileKmers + p.sym_base;
 }
 
-template <bool kDense>
+template <class C, bool kDense>
 __device__ __forceinline__ TileGeom tile_geom(const TileParams& p, uint64_t tile) {
     TileGeom g;
-    g.s0 = tile_first_symbol(p, tile);
+    g.s0 = tile_first_symbol<C>(p, tile);
     uint32_t need;
     if constexpr (kDense) {
         // 2-bit symbols: symbol s sits at bit 2s of the byte stream.
         g.b_lo = g.s0 >= 0 ? g.s0 / 4 : -((-g.s0 + 3) / 4);
-        need = (kCodeWords * 16 + 3) / 4 + 8;
+        need = (C::kCodeWords * 16 + 3) / 4 + 8;
     } else {
         g.b_lo = g.s0;
-        need = kCodeWords * 16 + 4;
+        need = C::kCodeWords * 16 + 4;
     }
     const uint64_t base = reinterpret_cast<uint64_t>(p.input);
     const uint64_t first = base + static_cast<uint64_t>(g.b_lo);  // wraps for b_lo < 0
@@ -114,10 +126,10 @@ __device__ __forceinline__ TileGeom tile_geom(const TileParams& p, uint64_t tile
 
 // Starts the tile's staging copy; returns whether it covers the whole stage
 // window (every tile but those at the input's ends).
-template <bool kDense>
+template <class C, bool kDense>
 __device__ __forceinline__ bool issue_stage(const TileParams& p, uint64_t tile, uint8_t* buf,
                                             uint64_t* bar) {
-    const TileGeom g = tile_geom<kDense>(p, tile);
+    const TileGeom g = tile_geom<C, kDense>(p, tile);
     fence_proxy_async_smem();
     if (g.hi > g.lo) {
         const uint32_t bytes = static_cast<uint32_t>(g.hi - g.lo);
@@ -160,13 +172,11 @@ __device__ __forceinline__ void fill_ragged(const TileParams& p, const TileGeom&
 
 // Where grid position 0 lies in the stage: its byte, or its bit for dense
 // input.  The same for every tile, since a tile is a multiple of 16 bytes.
-template <bool kDense>
+template <class C, bool kDense>
 __device__ __forceinline__ uint32_t stage_origin(const TileParams& p) {
-    const TileGeom g = tile_geom<kDense>(p, 0);
+    const TileGeom g = tile_geom<C, kDense>(p, 0);
     return kDense ? 8u * g.off + 2u * static_cast<uint32_t>(g.s0 - 4 * g.b_lo) : g.off;
 }
-static_assert(kTileKmers / 4 % 16 == 0, "tiles start at one phase of 16 bytes");
-
 // Encodes code word q (16 symbols from grid position 16q) of the staged tile.
 template <bool kDense>
 __device__ __forceinline__ void encode_word(uint32_t origin, const uint8_t* buf, int q,
@@ -252,7 +262,7 @@ __device__ __forceinline__ void sliding_min(const uint32_t* c, Fn&& fn) {
     }
 }
 
-// Calls fn(j, lo) for the strip's windows j = 0..kStrip-1 in order, lo being
+// Calls fn(j, lo) for the strip's windows in order, lo being
 // the low word of the window's minimum m-mer hash (its shard id, unmasked).
 // Windows of more than 16 m-mers take the minimum of their first and their
 // last 16.
@@ -261,13 +271,14 @@ __device__ __forceinline__ void for_each_min(const uint32_t* c, Fn&& fn) {
     constexpr int W = C::W;
     if constexpr (W == 1) {
 #pragma unroll
-        for (int j = 0; j < kStrip; ++j) fn(j, static_cast<uint32_t>(mh_at<C>(c, j)));
+        for (int j = 0; j < C::kStrip; ++j) fn(j, static_cast<uint32_t>(mh_at<C>(c, j)));
     } else if constexpr (W <= 16) {
-        sliding_min<C, W, kStrip>(c, [&](int j, uint64_t v) { fn(j, static_cast<uint32_t>(v)); });
+        sliding_min<C, W, C::kStrip>(
+            c, [&](int j, uint64_t v) { fn(j, static_cast<uint32_t>(v)); });
     } else {
         constexpr int D = W - 16;
         uint64_t first[D];
-        sliding_min<C, 16, kStrip + D>(c, [&](int j, uint64_t v) {
+        sliding_min<C, 16, C::kStrip + D>(c, [&](int j, uint64_t v) {
             if (j >= D) fn(j - D, static_cast<uint32_t>(min64(first[j % D], v)));
             first[j % D] = v;
         });
@@ -295,8 +306,10 @@ __device__ __forceinline__ uint64_t any_in_span(uint64_t x) {
 template <class C>
 __device__ __forceinline__ uint32_t strip_valid(uint64_t bits, int64_t first_kmer,
                                                 uint64_t n_kmers) {
-    uint32_t vmask = 0xFFFFFFFFu;
-    if (bits) vmask = ~static_cast<uint32_t>(any_in_span<C::K>(bits));
+    constexpr int kStrip = C::kStrip;
+    constexpr uint32_t kAll = 0xFFFFFFFFu >> (32 - kStrip);
+    uint32_t vmask = kAll;
+    if (bits) vmask = ~static_cast<uint32_t>(any_in_span<C::K>(bits)) & kAll;
     const int64_t left = static_cast<int64_t>(n_kmers) - first_kmer;  // windows from the first on
     if (first_kmer < 0) vmask = first_kmer > -kStrip ? vmask & (~0u << -first_kmer) : 0u;
     if (left < kStrip) vmask = left > 0 ? vmask & ((1u << left) - 1u) : 0u;
@@ -337,21 +350,23 @@ __device__ __forceinline__ void cp_async_wait_all() {
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
+// One byte per window; the grid phase aligns whole strips to their size.
+template <class C>
 __device__ __forceinline__ void store_strip_bytes(uint32_t result, uint8_t* out, int64_t first_kmer,
                                                   uint64_t n_kmers) {
+    constexpr int kStrip = C::kStrip;
     if (first_kmer >= 0 && first_kmer + kStrip <= static_cast<int64_t>(n_kmers)) {
-        uint4 v0, v1;
-        v0.x = spread4(result & 0xFu);
-        v0.y = spread4((result >> 4) & 0xFu);
-        v0.z = spread4((result >> 8) & 0xFu);
-        v0.w = spread4((result >> 12) & 0xFu);
-        v1.x = spread4((result >> 16) & 0xFu);
-        v1.y = spread4((result >> 20) & 0xFu);
-        v1.z = spread4((result >> 24) & 0xFu);
-        v1.w = spread4(result >> 28);
-        uint4* dst = reinterpret_cast<uint4*>(out + first_kmer);
-        dst[0] = v0;
-        dst[1] = v1;
+        uint32_t v[kStrip / 4];
+#pragma unroll
+        for (int q = 0; q < kStrip / 4; ++q) v[q] = spread4((result >> (4 * q)) & 0xFu);
+        if constexpr (kStrip == 8) {
+            *reinterpret_cast<uint2*>(out + first_kmer) = make_uint2(v[0], v[1]);
+        } else {
+            uint4* dst = reinterpret_cast<uint4*>(out + first_kmer);
+#pragma unroll
+            for (int q = 0; q < kStrip / 16; ++q)
+                dst[q] = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+        }
     } else {
 #pragma unroll
         for (int j = 0; j < kStrip; ++j) {
@@ -360,6 +375,20 @@ __device__ __forceinline__ void store_strip_bytes(uint32_t result, uint8_t* out,
                 out[i] = static_cast<uint8_t>((result >> j) & 1u);
         }
     }
+}
+
+// One bit per window (grid phase 0).  Strips up to the end of the last word
+// are written, so that its unused bits are 0.
+template <class C>
+__device__ __forceinline__ void store_strip_bits(uint32_t result, uint32_t* out,
+                                                 int64_t first_kmer, uint64_t n_kmers) {
+    if ((first_kmer & ~int64_t{31}) >= static_cast<int64_t>(n_kmers)) return;
+    if constexpr (C::kStrip == 32)
+        out[first_kmer >> 5] = result;
+    else if constexpr (C::kStrip == 16)
+        reinterpret_cast<uint16_t*>(out)[first_kmer >> 4] = static_cast<uint16_t>(result);
+    else
+        reinterpret_cast<uint8_t*>(out)[first_kmer >> 3] = static_cast<uint8_t>(result);
 }
 
 // Loads a slot's shard words x[0..7] from shared address `addr` when `pred` is
@@ -376,14 +405,34 @@ __device__ __forceinline__ void next_slot_if(uint32_t pred, uint32_t& addr, uint
         : "r"(pred));
 }
 
-// The strip's code words from shared address `at` (8-byte aligned).
-__device__ __forceinline__ void load_code_words(uint32_t at, uint32_t (&c)[kStripWords]) {
-    static_assert(kStripWords == 4, "two 8-byte loads");
-    asm volatile(
-        "ld.shared.v2.u32 {%0, %1}, [%4];\n\tld.shared.v2.u32 {%2, %3}, [%4+8];"
-        : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
-        : "r"(at)
-        : "memory");
+// The thread's strip of the tile's code words at shared address `code`: the
+// strip's first base comes to the top of c[0].
+template <class C>
+__device__ __forceinline__ void load_code_words(uint32_t code, uint32_t (&c)[kStripWords]) {
+    static_assert(kStripWords == 4, "four words");
+    const uint32_t tid = threadIdx.x;
+    if constexpr (C::kStrip == 32) {
+        asm volatile(
+            "ld.shared.v2.u32 {%0, %1}, [%4];\n\tld.shared.v2.u32 {%2, %3}, [%4+8];"
+            : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
+            : "r"(code + 8 * tid)
+            : "memory");
+    } else {
+        // 46 bases (16 windows of 31) are in three words.
+        const uint32_t at = code + (tid * C::kStrip / 16) * 4;
+        asm volatile(
+            "ld.shared.u32 %0, [%3];\n\tld.shared.u32 %1, [%3+4];\n\tld.shared.u32 %2, [%3+8];"
+            : "=r"(c[0]), "=r"(c[1]), "=r"(c[2])
+            : "r"(at)
+            : "memory");
+        c[3] = 0;
+        if constexpr (C::kStrip == 8) {
+            const uint32_t sh = 16 * (tid & 1u);
+            c[0] = __funnelshift_l(c[1], c[0], sh);
+            c[1] = __funnelshift_l(c[2], c[1], sh);
+            c[2] <<= sh;
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -457,10 +506,9 @@ __device__ __forceinline__ void copy_shards(uint32_t total, uint32_t pool, uint3
     cp_async_commit();
 }
 
-// Windows of one turn of the test pass.  The ring of a window's F s-mers keeps
-// position r at index r % F of the turn; turn() renames it for the next one.
+// The ring of a window's F s-mers keeps position r at index r % F of a turn of
+// 16 windows; turn() renames it for the next one.
 constexpr int kTurn = 16;
-static_assert(kStrip == 2 * kTurn, "two turns of one code word each");
 
 // Findere test of the window's F s-mers (F = 3 or 4) with byte permutes.  A bit
 // address is a byte n (upper three bits) and a bit t in it: for each shard
@@ -622,7 +670,7 @@ struct FindereTest<C, 1> {
 template <class C>
 __device__ __noinline__ uint3 list_runs(uint32_t code_mem, uint32_t list) {
     uint32_t c[kStripWords];
-    load_code_words(code_mem, c);
+    load_code_words<C>(code_mem, c);
     uint32_t at = list, chg = 1u, first = 0, prev = 0;
     for_each_min<C>(c, [&](int j, uint32_t lo) {
         if (j == 0) {
@@ -671,7 +719,7 @@ __device__ __forceinline__ uint32_t query_strip(uint32_t code_mem, uint32_t vmas
         const int n = __popc(heads);
         // A lane lends its last slot when that holds window 31's run and the run
         // is not its window 0's, which may itself be borrowed.
-        const bool lend = n > 0 && (vmask >> (kStrip - 1)) && !(n == 1 && (vmask & 1u));
+        const bool lend = n > 0 && (vmask >> (C::kStrip - 1)) && !(n == 1 && (vmask & 1u));
         const uint32_t left_lo = __shfl_up_sync(0xFFFFFFFFu, prev, 1);
         const uint32_t lenders = __ballot_sync(0xFFFFFFFFu, lend);
         const bool borrow =
@@ -701,7 +749,7 @@ __device__ __forceinline__ uint32_t query_strip(uint32_t code_mem, uint32_t vmas
         copy_shards(__reduce_max_sync(0xFFFFFFFFu, fits ? end : 0u), run_mem, ids, shard_mask,
                     words);
         uint32_t c[kStripWords];
-        load_code_words(code_mem, c);
+        load_code_words<C>(code_mem, c);
         typename FindereTest<C>::type test;
 #pragma unroll
         for (int o = 0; o < F - 1; ++o) test.enter(o, smer_hash(smer_at<C>(c, o)));
@@ -714,20 +762,24 @@ __device__ __forceinline__ uint32_t query_strip(uint32_t code_mem, uint32_t vmas
         // instructions of 32 unrolled windows, which ran out of the instruction
         // cache (10% of the stalls).
 #pragma unroll 1
-        for (int turn = 0; turn < 2; ++turn) {
+        for (int turn = 0; turn < C::kTurns; ++turn) {
             uint32_t m = 0;
 #pragma unroll
-            for (int j = 0; j < kTurn; ++j) {
+            for (int j = 0; j < C::kTurn; ++j) {
                 test.enter(j + F - 1, smer_hash(smer_at<C>(c, j + F - 1)));
                 next_slot_if(heads & (1u << j), at, x);
                 m += min(test.missing(x), 1u) << j;
             }
-            test.turn();
-            missing = (missing >> kTurn) | (m << kTurn);
-            heads >>= kTurn;
-            c[0] = c[1];
-            c[1] = c[2];
-            c[2] = c[3];
+            if constexpr (C::kTurns == 1) {
+                missing = m;
+            } else {
+                missing = (missing >> 16) | (m << 16);
+                test.turn();
+                heads >>= 16;
+                c[0] = c[1];
+                c[1] = c[2];
+                c[2] = c[3];
+            }
         }
         if (fits) {
             result |= vmask & ~missing;
@@ -749,7 +801,7 @@ __device__ __forceinline__ uint32_t query_strip_direct(uint32_t code_mem, uint32
                                                        const uint64_t* words) {
     constexpr int F = C::F;
     uint32_t c[kStripWords];
-    load_code_words(code_mem, c);
+    load_code_words<C>(code_mem, c);
     typename FindereTest<C>::type test;
 #pragma unroll
     for (int o = 0; o < F - 1; ++o) test.enter(o, smer_hash(smer_at<C>(c, o)));
@@ -879,7 +931,7 @@ __device__ __forceinline__ void insert_strip_runs(uint32_t code_mem, uint32_t vm
         const uint32_t chg = runs.x;
         uint32_t heads = vmask & (chg | ~(vmask << 1));
         const int n = __popc(heads);
-        const bool lend = n > 0 && (vmask >> (kStrip - 1)) && !(n == 1 && (vmask & 1u));
+        const bool lend = n > 0 && (vmask >> (C::kStrip - 1)) && !(n == 1 && (vmask & 1u));
         const uint32_t left_lo = __shfl_up_sync(0xFFFFFFFFu, runs.z, 1);
         const uint32_t lenders = __ballot_sync(0xFFFFFFFFu, lend);
         bool merge =
@@ -908,7 +960,7 @@ __device__ __forceinline__ void insert_strip_runs(uint32_t code_mem, uint32_t vm
         }
         __syncwarp();
         uint32_t c[kStripWords];
-        load_code_words(code_mem, c);
+        load_code_words<C>(code_mem, c);
         uint32_t ring[F][8];
         auto enter = [&](int r) {
             uint64_t m[4];
@@ -925,9 +977,9 @@ __device__ __forceinline__ void insert_strip_runs(uint32_t code_mem, uint32_t vm
         uint32_t at = merge ? spare : run_mem + 32 * begin;
         uint32_t next = run_mem + 32 * (merge ? begin : begin + 1);
 #pragma unroll 1
-        for (int turn = 0; turn < 2; ++turn) {
+        for (int turn = 0; turn < C::kTurns; ++turn) {
 #pragma unroll
-            for (int j = 0; j < kTurn; ++j) {
+            for (int j = 0; j < C::kTurn; ++j) {
                 enter(j + F - 1);
                 const uint32_t head = heads & (1u << j);
                 if constexpr (F == 4) {
@@ -946,6 +998,7 @@ __device__ __forceinline__ void insert_strip_runs(uint32_t code_mem, uint32_t vm
                 for (int q = 0; q < 8; ++q) acc[q] |= ring[(j + F - 1) % F][q];
                 store_run_if(ends & (1u << j), at, next, acc);
             }
+            if constexpr (C::kTurns == 1) break;
             heads >>= kTurn;
             ends >>= kTurn;
             c[0] = c[1];
@@ -987,7 +1040,7 @@ __device__ __forceinline__ void insert_strip_runs(uint32_t code_mem, uint32_t vm
 template <class C>
 __device__ __forceinline__ void mark_records(const TileParams& p, int64_t s0, uint32_t first,
                                              uint32_t* inval, uint32_t* brk) {
-    constexpr int64_t kSpan = kCodeWords * 16;
+    constexpr int64_t kSpan = C::kCodeWords * 16;
     const int64_t len = static_cast<int64_t>(p.input_bytes);
     const int64_t t_end = s0 + kSpan;
     auto set_bits = [&](uint32_t* arr, int64_t a, int64_t b) {  // dense [a, b)
@@ -1114,11 +1167,12 @@ __global__ void __launch_bounds__(kThreads, (kQuery ? query_three_ctas(C::W, C::
                                                 ? 3
                                                 : 2)
     tile_kernel(TileParams p) {
-    __shared__ alignas(128) uint8_t stage[kStageBytes];
+    constexpr int kCodeWords = C::kCodeWords;
+    __shared__ alignas(128) uint8_t stage[C::kStageBytes];
     __shared__ alignas(8) uint32_t code[kCodeWords + 4];
     // One bit per position: invalid bases, record starts.
-    __shared__ alignas(8) uint32_t inval[kCodeWords / 2 + 1];
-    __shared__ alignas(8) uint32_t brk[kRagged ? kCodeWords / 2 + 1 : 1];
+    __shared__ alignas(8) uint32_t inval[kCodeWords / 2 + 2];
+    __shared__ alignas(8) uint32_t brk[kRagged ? kCodeWords / 2 + 2 : 1];
     __shared__ uint64_t tiles[3];
     __shared__ uint32_t first_rec[3];
     __shared__ unsigned long long tally[2];
@@ -1154,7 +1208,7 @@ __global__ void __launch_bounds__(kThreads, (kQuery ? query_three_ctas(C::W, C::
         tally[0] = tally[1] = 0;
         const uint64_t t0 = take(0, 0);
         take(1, 1);
-        if (t0 < p.n_tiles) covered = issue_stage<kDense>(p, t0, stage, &bar);
+        if (t0 < p.n_tiles) covered = issue_stage<C, kDense>(p, t0, stage, &bar);
     }
     __syncthreads();
     // Dynamic shared memory: the query kernel's pool of shard slots, a part per
@@ -1162,7 +1216,7 @@ __global__ void __launch_bounds__(kThreads, (kQuery ? query_three_ctas(C::W, C::
     // [slot][thread] (kInsertSlotBytes per CTA).
     extern __shared__ __align__(16) uint64_t slots[];
     unsigned long long n_valid = 0, n_pos = 0;
-    const uint32_t origin = stage_origin<kDense>(p);
+    const uint32_t origin = stage_origin<C, kDense>(p);
     for (uint32_t it = 0;; ++it) {
         const uint64_t tile = tiles[it % 3];
         if (tile >= p.n_tiles) break;
@@ -1179,10 +1233,10 @@ __global__ void __launch_bounds__(kThreads, (kQuery ? query_three_ctas(C::W, C::
             return;
         }
         if (!covered) {
-            fill_ragged<kDense>(p, tile_geom<kDense>(p, tile), stage);
+            fill_ragged<kDense>(p, tile_geom<C, kDense>(p, tile), stage);
             __syncthreads();
         }
-        const int64_t s0 = tile_first_symbol(p, tile);
+        const int64_t s0 = tile_first_symbol<C>(p, tile);
         for (int q = tid; q < kCodeWords; q += kThreads) {
             uint32_t cw, iv;
             encode_word<kDense>(origin, stage, q, cw, iv);
@@ -1200,22 +1254,28 @@ __global__ void __launch_bounds__(kThreads, (kQuery ? query_three_ctas(C::W, C::
             // lands while this one is hashed.  The tile after it is taken now,
             // so that a barrier lies between its slot's write and its reads.
             const uint64_t next = tiles[(it + 1) % 3];
-            if (next < p.n_tiles) covered = issue_stage<kDense>(p, next, stage, &bar);
+            if (next < p.n_tiles) covered = issue_stage<C, kDense>(p, next, stage, &bar);
             take(it + 2, (it + 2) % 3);
         }
 
-        static_assert(kStrip == 32 && kStripWords == 4, "a strip's bits are two 32-bit words");
         auto strip_bits = [&](const uint32_t* a) {
-            return static_cast<uint64_t>(a[tid]) | (static_cast<uint64_t>(a[tid + 1]) << 32);
+            const uint32_t* w = a + (tid * C::kStrip) / 32;
+            if constexpr (C::kStrip == 32) {
+                return static_cast<uint64_t>(w[0]) | (static_cast<uint64_t>(w[1]) << 32);
+            } else {
+                const uint32_t sh = (tid * C::kStrip) & 31;
+                return static_cast<uint64_t>(__funnelshift_r(w[0], w[1], sh)) |
+                       (static_cast<uint64_t>(__funnelshift_r(w[1], w[2], sh)) << 32);
+            }
         };
-        const int64_t first_kmer = s0 + static_cast<int64_t>(tid) * kStrip;
+        const int64_t first_kmer = s0 + static_cast<int64_t>(tid) * C::kStrip;
         uint32_t vmask = strip_valid<C>(strip_bits(inval), first_kmer, p.n_kmers);
         if constexpr (kRagged) {
             vmask = strip_in_record<C>(strip_bits(brk), vmask);
             n_valid += __popc(vmask);
         }
         uint32_t hits = 0;
-        const uint32_t code_mem = smem_addr(code + tid * (kStrip / 16));
+        const uint32_t code_mem = smem_addr(code);
         if constexpr (kQuery) {
             if constexpr (C::W < 6 && C::M <= 8) {
                 hits = query_strip_direct<C>(code_mem, vmask, p.shard_mask, p.words);
@@ -1224,12 +1284,9 @@ __global__ void __launch_bounds__(kThreads, (kQuery ? query_three_ctas(C::W, C::
                 hits = query_strip<C>(code_mem, vmask, p.shard_mask, p.words,
                                       smem_addr(slots) + (tid >> 5) * kWarpBytes);
             }
-            if (p.out) store_strip_bytes(hits, p.out, first_kmer, p.n_kmers);
+            if (p.out) store_strip_bytes<C>(hits, p.out, first_kmer, p.n_kmers);
             if constexpr (kRagged) n_pos += __popc(hits & vmask);
-            // Bit-packed mode (grid phase 0, so strips start at multiples of
-            // 32 windows): one 32-bit word per strip, coalesced across the warp.
-            if (p.out_bits && first_kmer < static_cast<int64_t>(p.n_kmers))
-                p.out_bits[first_kmer >> 5] = hits;
+            if (p.out_bits) store_strip_bits<C>(hits, p.out_bits, first_kmer, p.n_kmers);
         } else {
             constexpr int kWarpBytes = insert_warp_bytes(C::W, C::H);
             insert_strip_runs<C>(code_mem, vmask, p.shard_mask, p.words,
