@@ -180,7 +180,7 @@ int sbf_filter::launch(bool query, bool dense, const void* input, uint64_t input
     p.gen = gen;
     const uint64_t resident = static_cast<uint64_t>(sms) * static_cast<uint64_t>(occupancy[which]);
     const uint64_t grid = std::min<uint64_t>(p.n_tiles, std::max<uint64_t>(resident, 1));
-    SBF_CUDA(launch_set_kernel(ks, kernel.fn, static_cast<unsigned>(grid), query, p, st));
+    SBF_CUDA(launch_set_kernel(ks, kernel.fn, static_cast<unsigned>(grid), which, p, st));
     ++launches;
     return SBF_OK;
 }
@@ -420,7 +420,7 @@ extern "C" int sbf_filter_create(uint32_t k, uint32_t s, uint32_t m, uint32_t ha
         // answer, the set's assumption (two CTAs per SM for the tile
         // kernels, as their shared memory allows) stands.
         for (int i = 0; i < 6 && ks->jit; ++i) {
-            const int dyn = ks->smem((i & 1) != 0);
+            const int dyn = ks->smem(i);
             int occ = 0;
             if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fns[i], kThreads, dyn) !=
                     cudaSuccess ||
@@ -432,7 +432,7 @@ extern "C" int sbf_filter_create(uint32_t k, uint32_t s, uint32_t m, uint32_t ha
         }
         for (int i = 0; i < 6 && rc == SBF_OK && !ks->jit; ++i) {
             // Query kernels: shard slots; insert kernels: flush staging ring.
-            const int dyn = ks->smem((i & 1) != 0);
+            const int dyn = ks->smem(i);
             if (dyn) {
                 e = cudaFuncSetAttribute(reinterpret_cast<const void*>(fns[i]),
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, dyn);

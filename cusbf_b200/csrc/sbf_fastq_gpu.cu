@@ -670,7 +670,7 @@ int FastqDevice::launch_block_graph(sbf_filter* f, bool query, bool fasta, const
             return r;
         TileParams copy = p;
         void* args[] = {&copy};
-        if ((r = cudaLaunchKernel(tile_fn, dim3(tile_grid), dim3(kThreads), args, f->ks->smem(query),
+        if ((r = cudaLaunchKernel(tile_fn, dim3(tile_grid), dim3(kThreads), args, f->ks->smem(query ? kQueryRagged : kInsertRagged),
                                   st)) != cudaSuccess)
             return r;
         if ((r = cudaMemcpyAsync(reinterpret_cast<uint8_t*>(h_summary.p) + offsetof(BlockSummary, valid),

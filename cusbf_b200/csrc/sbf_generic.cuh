@@ -1,7 +1,8 @@
-// sbf_generic.cuh -- runtime-parameterised insert / query kernels for every
-// configuration that has no specialised tile kernel: any k, s, m and hash
-// count the reference's Config accepts (config.cuh:28-118), and the protein
-// and DNA-triplet alphabets (Alphabet.cuh:150-220).
+// sbf_generic.cuh -- runtime-parameterised insert / query kernels for whatever
+// has no tile kernel: DNA triplets, dense proteins and proteins with short
+// windows (sbf_jit.cpp), and, where nothing can be compiled at run time, any
+// k, s, m and hash count the reference's Config accepts (config.cuh:28-118)
+// and every alphabet (Alphabet.cuh:150-220).
 //
 // Each thread owns a strip of 32 consecutive windows.  The strip's k-mer is
 // packed MSB-first and slid one symbol per window
@@ -260,9 +261,9 @@ __global__ void __launch_bounds__(kThreads) generic_kernel(TileParams p) {
             // its newest m-mer and s-mer, kept in rings of the window's W
             // m-mer hashes and F s-mer masks (slot x % W holds the m-mer
             // starting at symbol w0 + x).  The strip is unrolled, so ring
-            // slots are registers.  (Protein <12,10,6,4>: insert 72.8 -> 76.9
-            // G windows/s; the same form made the query 16% slower, so
-            // queries evaluate each window whole.)
+            // slots are registers.  (Protein <12,10,6,4>, before it had tile
+            // kernels: insert 72.8 -> 76.9 G windows/s; the same form made the
+            // query 16% slower, so queries evaluate each window whole.)
             constexpr int kK = G::kK, kM = G::kM, kS = G::kS, kBits = G::kBits;
             constexpr int W = kK - kM + 1, F = kK - kS + 1;
             const uint64_t mm_mask = low_mask(kM * kBits);

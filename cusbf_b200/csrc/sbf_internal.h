@@ -42,7 +42,7 @@ SBF_SIZE_FN int query_cta_bytes(int w, int h) { return kThreads / 32 * query_war
 // masks, and a spare slot per lane for a run that a neighbour flushes.  184
 // slots leave room for three CTAs and 4 deviations at W = 12 (158 slots).
 SBF_SIZE_FN bool insert_three_ctas(int w, int h) { return w >= 12 && w <= 16 && h <= 8; }
-SBF_SIZE_FN int insert_pool_slots(int w, int h) { return insert_three_ctas(w, h) ? 184 : 320; }
+SBF_SIZE_FN int insert_pool_slots(int w, int h) { return insert_three_ctas(w, h) ? 184 : 312; }
 SBF_SIZE_FN int insert_warp_bytes(int w, int h) {
     return insert_pool_slots(w, h) * (32 + 4) + 32 * 32;
 }
@@ -139,7 +139,13 @@ struct KernelSet {
                                     query_dense,  insert_ragged, query_ragged};
         return fns[which];
     }
-    int smem(bool query) const { return query ? smem_query : smem_insert; }
+    // Protein tile sets: the dense kernels are the generic ones.
+    bool generic_dense = false;
+    int smem(int which) const {
+        const bool query = (which & 1) != 0;
+        if (generic_dense && (which == 2 || which == 3)) return query ? 0 : kInsertSlotBytes;
+        return query ? smem_query : smem_insert;
+    }
 };
 
 // Which of a set's kernels: insert or query of bytes, dense words, records.
@@ -177,12 +183,12 @@ cudaError_t launch_tile_records_sized(const DevRange* ranges, const DevSizes* si
 cudaError_t launch_popcount(const uint64_t* words, uint64_t n_words, unsigned long long* out,
                             cudaStream_t stream);
 // Kernels compiled at run time for a configuration that is not compiled into
-// the library (sbf_jit.cpp): the tile kernels for DNA, the generic kernels
-// with the configuration as constants for the other alphabets; nullptr when
-// that is not possible.
+// the library (sbf_jit.cpp): the tile kernels for DNA and proteins, the generic
+// kernels with the configuration as constants for the rest; nullptr when that
+// is not possible.
 const KernelSet* jit_kernels(int k, int s, int m, int h, int alphabet, int device);
 // Launches one of a KernelSet's kernels.
-cudaError_t launch_set_kernel(const KernelSet* ks, const void* fn, unsigned grid, bool query,
+cudaError_t launch_set_kernel(const KernelSet* ks, const void* fn, unsigned grid, int which,
                               const TileParams& p, cudaStream_t stream);
 #endif
 

@@ -10,9 +10,9 @@
 // Compilation takes about ten seconds, so the cubin is cached on disk under
 // $SBF_JIT_CACHE (default ~/.cache/sbf_b200), keyed by the configuration, the
 // device architecture, the NVRTC version and a hash of the embedded source.
-// The protein and DNA-triplet alphabets get the generic kernels
-// (sbf_generic.cuh) compiled the same way with the configuration as template
-// constants.  SBF_JIT=0 turns this off; then, and on any failure, the filter
+// Proteins get the tile kernels as well (JitConfig::tile); DNA triplets and
+// dense proteins get the generic kernels (sbf_generic.cuh) compiled the same
+// way with the configuration as template constants.  SBF_JIT=0 turns this off; then, and on any failure, the filter
 // runs the runtime-parameterised generic kernels, which give the same
 // results more slowly.
 #include <cuda_runtime.h>
@@ -139,19 +139,27 @@ struct Compiled {
     std::vector<char> cubin;
 };
 
-// One configuration to compile: DNA gets the tile kernels, other alphabets
-// the generic kernels with the configuration as template constants.
+// One configuration to compile: the tile kernels where the alphabet has them,
+// else the generic kernels with the configuration as template constants.
 struct JitConfig {
     int k, s, m, h, alphabet;
     uint32_t bits, width;
-    bool tile() const { return alphabet == SBF_ALPHABET_DNA; }
+    // Variant v (kVariants) gets a tile kernel: all of DNA's, and a protein
+    // configuration's but the dense ones and those with windows of less than 4
+    // m-mers, whose pools take several rounds (64 M windows of <8,6,8,4>, one
+    // m-mer: query 1.05 ms in the tile kernel, 0.61 in the generic one;
+    // <12,10,6,4>, seven: 0.29 and 0.65).
+    bool tile(int v) const {
+        return alphabet == SBF_ALPHABET_DNA ||
+               (alphabet == SBF_ALPHABET_PROTEIN && !kVariants[v][1] && k - m >= 3);
+    }
 };
 
 std::string name_expr(const JitConfig& c, int v) {
     char cfg[96], buf[192];
-    if (c.tile())
-        std::snprintf(cfg, sizeof cfg, "sbf::tile_kernel<sbf::Cfg<%d, %d, %d, %d>", c.k, c.s, c.m,
-                      c.h);
+    if (c.tile(v))
+        std::snprintf(cfg, sizeof cfg, "sbf::tile_kernel<sbf::Cfg<%d, %d, %d, %d, sbf::kStrip, %u>",
+                      c.k, c.s, c.m, c.h, c.bits);
     else
         std::snprintf(cfg, sizeof cfg, "sbf::generic_kernel<sbf::FixedGen<%d, %d, %d, %d, %u, %u, %d>",
                       c.k, c.s, c.m, c.h, c.bits, c.width, c.alphabet);
@@ -166,8 +174,8 @@ bool compile(const JitConfig& c, const std::string& arch, Compiled* out) {
     const char* headers[] = {kJitInternal, kJitDevice, kJitFlush, kJitTile, kJitGeneric};
     const char* names[] = {"sbf_internal.h", "sbf_device.cuh", "sbf_flush.cuh", "sbf_tile.cuh",
                            "sbf_generic.cuh"};
-    const std::string src = std::string(kPrelude) +
-                            (c.tile() ? "#include \"sbf_tile.cuh\"\n" : "#include \"sbf_generic.cuh\"\n");
+    const std::string src = std::string(kPrelude) + (c.tile(0) ? "#include \"sbf_tile.cuh\"\n" : "") +
+                            (c.tile(2) ? "" : "#include \"sbf_generic.cuh\"\n");
     nvrtcProgram prog;
     if (nv.create(&prog, src.c_str(), "sbf_jit.cu", 5, headers, names) != NVRTC_SUCCESS)
         return false;
@@ -276,7 +284,7 @@ const KernelSet* jit_kernels(int k, int s, int m, int h, int alphabet, int devic
         hash = fnv1a(hash, arch.data(), arch.size());
         char file[128];
         std::snprintf(file, sizeof file, "%s_k%d_s%d_m%d_h%d_a%d_%016llx.bin",
-                      jc.tile() ? "tile" : "generic", k, s, m, h, alphabet,
+                      jc.tile(0) ? "tile" : "generic", k, s, m, h, alphabet,
                       static_cast<unsigned long long>(hash));
         const std::string dir = cache_dir();
         const std::string path = dir + "/" + file;
@@ -309,7 +317,9 @@ const KernelSet* jit_kernels(int k, int s, int m, int h, int alphabet, int devic
         }
         e->ks = KernelSet{k, s, m, h, fns[0], fns[1], fns[2], fns[3], fns[4], fns[5]};
         e->ks.jit = true;
-        if (!jc.tile()) {
+        if (jc.tile(0)) {
+            e->ks.generic_dense = !jc.tile(2);
+        } else {
             // The generic kernels use few registers; inserts take the flush
             // ring's dynamic shared memory, queries none.
             e->ks.smem_insert = kInsertSlotBytes;
@@ -323,7 +333,7 @@ const KernelSet* jit_kernels(int k, int s, int m, int h, int alphabet, int devic
         const void* fns[6] = {e.ks.insert_bytes, e.ks.query_bytes,   e.ks.insert_dense,
                               e.ks.query_dense,  e.ks.insert_ragged, e.ks.query_ragged};
         for (int v = 0; v < 6; ++v) {
-            const int dyn = e.ks.smem(kVariants[v][0]);
+            const int dyn = e.ks.smem(v);
             if (dyn == 0) continue;
             if (cudaKernelSetAttributeForDevice(
                     reinterpret_cast<cudaKernel_t>(const_cast<void*>(fns[v])),

@@ -190,7 +190,7 @@ StripKernel strip_kernel(const KernelSet* ks, int which, uint64_t n_kmers, int d
     std::atomic<uint64_t>& devices = ready[config][strip == 16][which];
     if (!(devices.load(std::memory_order_acquire) >> device & 1u)) {
         if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 ks->smem((which & 1) != 0)) != cudaSuccess) {
+                                 ks->smem(which)) != cudaSuccess) {
             cudaGetLastError();
             return own;
         }
@@ -199,11 +199,11 @@ StripKernel strip_kernel(const KernelSet* ks, int which, uint64_t n_kmers, int d
     return {fn, strip};
 }
 
-cudaError_t launch_set_kernel(const KernelSet* ks, const void* fn, unsigned grid, bool query,
+cudaError_t launch_set_kernel(const KernelSet* ks, const void* fn, unsigned grid, int which,
                               const TileParams& p, cudaStream_t stream) {
     TileParams copy = p;
     void* args[] = {&copy};
-    return cudaLaunchKernel(fn, dim3(grid), dim3(kThreads), args, ks->smem(query), stream);
+    return cudaLaunchKernel(fn, dim3(grid), dim3(kThreads), args, ks->smem(which), stream);
 }
 
 }  // namespace sbf

@@ -215,11 +215,13 @@ static unsigned ragged_grid(const sbf_filter* f, bool query, uint64_t n_tiles, u
 int ragged_launch(sbf_filter* f, bool query, const TileParams& p, uint32_t ctas,
                   cudaStream_t st, StripKernel kernel) {
     if (p.n_tiles == 0) return SBF_OK;
-    if (!kernel.fn) kernel = {f->ks->fn(query ? kQueryRagged : kInsertRagged), kStrip};
+    const int which = query ? kQueryRagged : kInsertRagged;
+    if (!kernel.fn) kernel = {f->ks->fn(which), kStrip};
     SBF_CUDA(launch_tile_records(p.ranges, p.n_ranges, p.sym_base, kernel.tile_kmers(), p.n_tiles,
                                  const_cast<uint32_t*>(p.tile_rec), st));
     SBF_CUDA(cudaMemsetAsync(p.queue, 0, sizeof(unsigned int), st));
-    SBF_CUDA(launch_set_kernel(f->ks, kernel.fn, ragged_grid(f, query, p.n_tiles, ctas), query, p, st));
+    SBF_CUDA(launch_set_kernel(f->ks, kernel.fn, ragged_grid(f, query, p.n_tiles, ctas),
+                               which, p, st));
     f->launches += 2;
     return SBF_OK;
 }
@@ -250,7 +252,7 @@ int ragged_graph_launch(sbf_filter* f, RaggedGraph& g, bool query, const TilePar
     tk.func = const_cast<void*>(query ? f->ks->query_ragged : f->ks->insert_ragged);
     tk.gridDim = dim3(ragged_grid(f, query, p.n_tiles, ctas));
     tk.blockDim = dim3(kThreads);
-    tk.sharedMemBytes = f->ks->smem(query);
+    tk.sharedMemBytes = f->ks->smem(query ? kQueryRagged : kInsertRagged);
     tk.kernelParams = tile_args;
     if (!g.exec) {
         SBF_CUDA(cudaGraphCreate(&g.graph, 0));

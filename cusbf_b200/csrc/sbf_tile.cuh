@@ -1,7 +1,7 @@
 // sbf_tile.cuh -- sm_100a insert / query tile kernels of the Super Bloom engine
 // (device code only: compiled into the library for the common configurations
-// by sbf_kernels.cu, and for any other DNA configuration at run time by
-// sbf_jit.cpp).
+// by sbf_kernels.cu and sbf_narrow*.cu, and for any other DNA configuration
+// and for proteins at run time by sbf_jit.cpp).
 //
 // Reference path replaced: include/cusbf/detail/kernels.cuh:179-312 of
 // tdortman/cuSBF (insert_sequence_kmers_kernel, contains_sequence_kmers_kernel
@@ -45,8 +45,9 @@
 
 namespace sbf {
 
-// A filter configuration and the windows per thread (strip).
-template <int K_, int S_, int M_, int H_, int Strip_ = kStrip>
+// A filter configuration, the windows per thread (strip) and the bits of a
+// symbol: 2 for DNA, 5 for proteins.
+template <int K_, int S_, int M_, int H_, int Strip_ = kStrip, int Bits_ = 2>
 struct Cfg {
     static constexpr int K = K_;
     static constexpr int S = S_;
@@ -54,16 +55,24 @@ struct Cfg {
     static constexpr int H = H_;
     static constexpr int W = K - M + 1;  // m-mers per window
     static constexpr int F = K - S + 1;  // s-mers per window (findere span)
+    static constexpr int kBits = Bits_;
     static constexpr int kStrip = Strip_;
     static constexpr int kTileKmers = kThreads * kStrip;
-    static constexpr int kCodeWords = (kThreads - 1) * kStrip / 16 + kStripWords;
-    static constexpr int kStageBytes = kCodeWords * 16 + 64;
+    // Code words of a strip and of a tile.  DNA words hold 16 bases; protein
+    // symbols run on from word to word, five words a strip.
+    static constexpr int kStripWords =
+        kBits == 2 ? sbf::kStripWords : ((kStrip + K - 1) * kBits + 31) / 32;
+    static constexpr int kCodeWords = kBits == 2 ? (kThreads - 1) * kStrip / 16 + kStripWords
+                                                 : (kThreads + 1) * kStrip * kBits / 32;
+    static constexpr int kSpan = kCodeWords * 32 / kBits;  // symbols staged and encoded
+    static constexpr int kStageBytes = kSpan + 64;
     // The passes over a strip's windows take them in turns of at most 16.
     static constexpr int kTurn = kStrip < 16 ? kStrip : 16;
     static constexpr int kTurns = kStrip / kTurn;
     static_assert(kStrip == 8 || kStrip == 16 || kStrip == 32, "strips of 8, 16 or 32 windows");
     static_assert(kTileKmers / 4 % 16 == 0, "tiles start at one phase of 16 bytes");
-    static_assert(K >= 1 && K <= 32, "k must fit a 64-bit packed window");
+    static_assert(kBits == 2 || (kBits == 5 && kStrip == 32), "DNA, or proteins in full strips");
+    static_assert(K >= 1 && K * kBits <= 64, "k must fit a 64-bit packed window");
     static_assert(M >= 1 && M <= K, "m must satisfy 1 <= m <= k");
     static_assert(S >= 1 && S <= K, "s must satisfy 1 <= s <= k");
     static_assert(H % 4 == 0 && H >= 4 && H <= 16, "hash count must be 4, 8, 12 or 16");
@@ -99,7 +108,7 @@ __device__ __forceinline__ TileGeom tile_geom(const TileParams& p, uint64_t tile
         need = (C::kCodeWords * 16 + 3) / 4 + 8;
     } else {
         g.b_lo = g.s0;
-        need = C::kCodeWords * 16 + 4;
+        need = C::kSpan + 4;
     }
     const uint64_t base = reinterpret_cast<uint64_t>(p.input);
     const uint64_t first = base + static_cast<uint64_t>(g.b_lo);  // wraps for b_lo < 0
@@ -199,6 +208,41 @@ __device__ __forceinline__ void encode_word(uint32_t origin, const uint8_t* buf,
     }
 }
 
+// Encodes the 32 protein symbols from grid position 32 t into five code words
+// (5 bits a symbol, earliest symbol in the top bits) and a word of invalid
+// bits.  Letters only, either case; code = letter - 'A'.  With the rest of the
+// tile kernel as for DNA, 64 M residues of <12,10,6,4> take 287 us to query and
+// 362 to insert, where a byte load and a whole window's hashes per window took
+// 647 and 736 (sbf_generic.cuh).
+__device__ __forceinline__ void encode_protein_strip(uint32_t origin, const uint8_t* buf, int t,
+                                                     uint32_t* code, uint32_t* inval) {
+    const uint32_t bytepos = origin + 32u * t;
+    const uint32_t* x = reinterpret_cast<const uint32_t*>(buf) + (bytepos >> 2);
+    const uint32_t sh = (bytepos & 3u) * 8u;
+    uint32_t g[8], bad[8], any = 0;  // 20 bits of four symbols, their invalid bytes
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const uint32_t v = __funnelshift_r(x[i], x[i + 1], sh);
+        const uint32_t c = ((v & 0x1F1F1F1Fu) + 0x1F1F1F1Fu) & 0x1F1F1F1Fu;
+        // Above 'Z' (code 26 and up, '@' wraps to 31), or not 01xxxxxx.
+        bad[i] = ((c + 0x66666666u) & 0x80808080u) | ((v ^ 0x40404040u) & 0xC0C0C0C0u);
+        any |= bad[i];
+        const uint32_t pair = (c & 0x001F001Fu) * 32u + ((c >> 8) & 0x001F001Fu);
+        g[i] = (pair & 0xFFFFu) * 1024u + (pair >> 16);
+    }
+    code[5 * t] = (g[0] << 12) | (g[1] >> 8);
+    code[5 * t + 1] = (g[1] << 24) | (g[2] << 4) | (g[3] >> 16);
+    code[5 * t + 2] = (g[3] << 16) | (g[4] >> 4);
+    code[5 * t + 3] = (g[4] << 28) | (g[5] << 8) | (g[6] >> 12);
+    code[5 * t + 4] = (g[6] << 20) | g[7];
+    uint32_t bits = 0;
+    if (any) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) bits |= nonzero_bytes_to_bits(bad[i]) << (4 * i);
+    }
+    inval[t] = bits;
+}
+
 // Expands the four low bits of `nib` into four 0/1 bytes (bit r -> byte r).
 __device__ __forceinline__ uint32_t spread4(uint32_t nib) {
     return (nib * 0x00204081u) & 0x01010101u;
@@ -208,33 +252,40 @@ __device__ __forceinline__ uint32_t spread4(uint32_t nib) {
 // Strip computation: kStrip consecutive windows per thread
 // ---------------------------------------------------------------------------
 
-// The 16 bases starting at strip position r, earliest base in bits 31:30.
-// `c` holds the strip's code words; r is a compile-time constant after
-// unrolling, so every access is a register.
-__device__ __forceinline__ uint32_t win16(const uint32_t* c, int r) {
-    const int q = r >> 4, s = r & 15;
-    return s == 0 ? c[q] : __funnelshift_l(c[q + 1], c[q], 2 * s);
+// The 32 bits from bit `at` of the strip's code words (earliest bits on top).
+// `at` is a compile-time constant after unrolling, so every access is a
+// register; bits past the last word read 0.
+template <class C>
+__device__ __forceinline__ uint32_t bits32(const uint32_t* c, int at) {
+    const int q = at >> 5, s = at & 31;
+    if (s == 0) return c[q];
+    return __funnelshift_l(q + 1 < C::kStripWords ? c[q + 1] : 0u, c[q], s);
 }
 
+// The `bits` bits from bit `at` on, right-aligned.
+template <class C, int bits>
+__device__ __forceinline__ uint64_t bits64(const uint32_t* c, int at) {
+    if constexpr (bits > 32) {
+        const uint64_t hi = bits32<C>(c, at) >> (64 - bits);
+        return (hi << 32) | bits32<C>(c, at + bits - 32);
+    } else {
+        return bits32<C>(c, at) >> (32 - bits);
+    }
+}
+
+// The hash of the m-mer, and the s-mer, at strip position r.
 template <class C>
 __device__ __forceinline__ uint64_t mh_at(const uint32_t* c, int r) {
-    if constexpr (C::M > 16) {
-        // Longer m-mers span two 16-base windows, like long s-mers.
-        const uint64_t hi = win16(c, r) >> (2 * (32 - C::M));
-        return mmer_hash((hi << 32) | win16(c, r + C::M - 16));
-    } else {
-        return mmer_hash(win16(c, r) >> (2 * (16 - C::M)));
-    }
+    const uint64_t v = bits64<C, C::M * C::kBits>(c, r * C::kBits);
+    if constexpr (C::M * C::kBits > 32)
+        return mmer_hash(v);
+    else
+        return mmer_hash(static_cast<uint32_t>(v));
 }
 
 template <class C>
 __device__ __forceinline__ uint64_t smer_at(const uint32_t* c, int r) {
-    if constexpr (C::S > 16) {
-        const uint64_t hi = win16(c, r) >> (2 * (32 - C::S));
-        return (hi << 32) | win16(c, r + C::S - 16);
-    } else {
-        return win16(c, r) >> (2 * (16 - C::S));
-    }
+    return bits64<C, C::S * C::kBits>(c, r * C::kBits);
 }
 
 // Calls fn(j, v) for j = 0..N-1 in order, v being the minimum hash of the W
@@ -391,6 +442,22 @@ __device__ __forceinline__ void store_strip_bits(uint32_t result, uint32_t* out,
         reinterpret_cast<uint8_t*>(out)[first_kmer >> 3] = static_cast<uint8_t>(result);
 }
 
+// Windows of a turn of a strip of 32.  The ring of a window's F s-mers keeps
+// position r at index r % F of the turn; its turn() renames it for the next.
+constexpr int kTurn = 16;
+
+// Moves the strip's code words on by the 16 windows of a turn.
+template <class C>
+__device__ __forceinline__ void next_turn_words(uint32_t (&c)[C::kStripWords]) {
+    constexpr int kWords = kTurn * C::kBits / 32, kShift = kTurn * C::kBits % 32;
+#pragma unroll
+    for (int q = 0; q < C::kStripWords; ++q) {
+        const uint32_t a = q + kWords < C::kStripWords ? c[q + kWords] : 0u;
+        const uint32_t b = q + kWords + 1 < C::kStripWords ? c[q + kWords + 1] : 0u;
+        c[q] = kShift ? __funnelshift_l(b, a, kShift) : a;
+    }
+}
+
 // Loads a slot's shard words x[0..7] from shared address `addr` when `pred` is
 // non-zero, leaves them unchanged otherwise, and advances `addr` to the next
 // slot after a load: predicated, so that a run head costs no branch.
@@ -408,10 +475,16 @@ __device__ __forceinline__ void next_slot_if(uint32_t pred, uint32_t& addr, uint
 // The thread's strip of the tile's code words at shared address `code`: the
 // strip's first base comes to the top of c[0].
 template <class C>
-__device__ __forceinline__ void load_code_words(uint32_t code, uint32_t (&c)[kStripWords]) {
-    static_assert(kStripWords == 4, "four words");
+__device__ __forceinline__ void load_code_words(uint32_t code, uint32_t (&c)[C::kStripWords]) {
     const uint32_t tid = threadIdx.x;
-    if constexpr (C::kStrip == 32) {
+    if constexpr (C::kBits != 2) {
+#pragma unroll
+        for (int q = 0; q < C::kStripWords; ++q)
+            asm volatile("ld.shared.u32 %0, [%1];"
+                         : "=r"(c[q])
+                         : "r"(code + (C::kStrip * C::kBits / 8) * tid + 4 * q)
+                         : "memory");
+    } else if constexpr (C::kStrip == 32) {
         asm volatile(
             "ld.shared.v2.u32 {%0, %1}, [%4];\n\tld.shared.v2.u32 {%2, %3}, [%4+8];"
             : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
@@ -506,9 +579,6 @@ __device__ __forceinline__ void copy_shards(uint32_t total, uint32_t pool, uint3
     cp_async_commit();
 }
 
-// The ring of a window's F s-mers keeps position r at index r % F of a turn of
-// 16 windows; turn() renames it for the next one.
-constexpr int kTurn = 16;
 
 // Findere test of the window's F s-mers (F = 3 or 4) with byte permutes.  A bit
 // address is a byte n (upper three bits) and a bit t in it: for each shard
@@ -669,7 +739,7 @@ struct FindereTest<C, 1> {
 // kernel's.
 template <class C>
 __device__ __noinline__ uint3 list_runs(uint32_t code_mem, uint32_t list) {
-    uint32_t c[kStripWords];
+    uint32_t c[C::kStripWords];
     load_code_words<C>(code_mem, c);
     uint32_t at = list, chg = 1u, first = 0, prev = 0;
     for_each_min<C>(c, [&](int j, uint32_t lo) {
@@ -748,7 +818,7 @@ __device__ __forceinline__ uint32_t query_strip(uint32_t code_mem, uint32_t vmas
         __syncwarp();
         copy_shards(__reduce_max_sync(0xFFFFFFFFu, fits ? end : 0u), run_mem, ids, shard_mask,
                     words);
-        uint32_t c[kStripWords];
+        uint32_t c[C::kStripWords];
         load_code_words<C>(code_mem, c);
         typename FindereTest<C>::type test;
 #pragma unroll
@@ -776,9 +846,7 @@ __device__ __forceinline__ uint32_t query_strip(uint32_t code_mem, uint32_t vmas
                 missing = (missing >> 16) | (m << 16);
                 test.turn();
                 heads >>= 16;
-                c[0] = c[1];
-                c[1] = c[2];
-                c[2] = c[3];
+                next_turn_words<C>(c);
             }
         }
         if (fits) {
@@ -800,7 +868,7 @@ __device__ __forceinline__ uint32_t query_strip_direct(uint32_t code_mem, uint32
                                                        uint32_t shard_mask,
                                                        const uint64_t* words) {
     constexpr int F = C::F;
-    uint32_t c[kStripWords];
+    uint32_t c[C::kStripWords];
     load_code_words<C>(code_mem, c);
     typename FindereTest<C>::type test;
 #pragma unroll
@@ -879,7 +947,7 @@ __device__ __forceinline__ void or_slot(uint32_t dst, uint32_t src) {
 // bulk reduction per slot takes 72 G slots/s from an L2-resident filter where
 // this takes 120, and both 20 to 31 G/s from larger ones.  It also holds the
 // slot until it is read.)
-__device__ __forceinline__ void flush_slots(uint32_t total, uint32_t pool, uint32_t ids,
+__device__ __forceinline__ void flush_pool(uint32_t total, uint32_t pool, uint32_t ids,
                                             uint32_t shard_mask, uint64_t* words) {
     const uint32_t lane = threadIdx.x & 31;
     uint64_t* word = words + (lane & 3u);
@@ -959,7 +1027,7 @@ __device__ __forceinline__ void insert_strip_runs(uint32_t code_mem, uint32_t vm
             copy_u32_if(b, at, list + 128 * e);
         }
         __syncwarp();
-        uint32_t c[kStripWords];
+        uint32_t c[C::kStripWords];
         load_code_words<C>(code_mem, c);
         uint32_t ring[F][8];
         auto enter = [&](int r) {
@@ -1001,9 +1069,7 @@ __device__ __forceinline__ void insert_strip_runs(uint32_t code_mem, uint32_t vm
             if constexpr (C::kTurns == 1) break;
             heads >>= kTurn;
             ends >>= kTurn;
-            c[0] = c[1];
-            c[1] = c[2];
-            c[2] = c[3];
+            next_turn_words<C>(c);
             if constexpr (kTurn % F != 0) {
                 uint32_t old[F][8];
 #pragma unroll
@@ -1021,7 +1087,7 @@ __device__ __forceinline__ void insert_strip_runs(uint32_t code_mem, uint32_t vm
         __syncwarp();
         if (merge) or_slot(run_mem + 32 * (begin - 1), spare);
         __syncwarp();
-        flush_slots(__reduce_max_sync(0xFFFFFFFFu, fits ? end : 0u), run_mem, ids, shard_mask,
+        flush_pool(__reduce_max_sync(0xFFFFFFFFu, fits ? end : 0u), run_mem, ids, shard_mask,
                     words);
         __syncwarp();  // the slots are read before another round's lists replace them
         if (fits) vmask = 0;
@@ -1040,7 +1106,7 @@ __device__ __forceinline__ void insert_strip_runs(uint32_t code_mem, uint32_t vm
 template <class C>
 __device__ __forceinline__ void mark_records(const TileParams& p, int64_t s0, uint32_t first,
                                              uint32_t* inval, uint32_t* brk) {
-    constexpr int64_t kSpan = C::kCodeWords * 16;
+    constexpr int64_t kSpan = C::kSpan;
     const int64_t len = static_cast<int64_t>(p.input_bytes);
     const int64_t t_end = s0 + kSpan;
     auto set_bits = [&](uint32_t* arr, int64_t a, int64_t b) {  // dense [a, b)
@@ -1171,8 +1237,8 @@ __global__ void __launch_bounds__(kThreads, (kQuery ? query_three_ctas(C::W, C::
     __shared__ alignas(128) uint8_t stage[C::kStageBytes];
     __shared__ alignas(8) uint32_t code[kCodeWords + 4];
     // One bit per position: invalid bases, record starts.
-    __shared__ alignas(8) uint32_t inval[kCodeWords / 2 + 2];
-    __shared__ alignas(8) uint32_t brk[kRagged ? kCodeWords / 2 + 2 : 1];
+    __shared__ alignas(8) uint32_t inval[C::kSpan / 32 + 2];
+    __shared__ alignas(8) uint32_t brk[kRagged ? C::kSpan / 32 + 2 : 1];
     __shared__ uint64_t tiles[3];
     __shared__ uint32_t first_rec[3];
     __shared__ unsigned long long tally[2];
@@ -1237,7 +1303,14 @@ __global__ void __launch_bounds__(kThreads, (kQuery ? query_three_ctas(C::W, C::
             __syncthreads();
         }
         const int64_t s0 = tile_first_symbol<C>(p, tile);
-        for (int q = tid; q < kCodeWords; q += kThreads) {
+        if constexpr (C::kBits != 2) {
+            static_assert(!kDense || C::kBits == 2, "dense proteins run the generic kernels");
+            for (int t = tid; t <= kThreads; t += kThreads) {
+                encode_protein_strip(origin, stage, t, code, inval);
+                if constexpr (kRagged) brk[t] = 0u;
+            }
+        }
+        for (int q = tid; C::kBits == 2 && q < kCodeWords; q += kThreads) {
             uint32_t cw, iv;
             encode_word<kDense>(origin, stage, q, cw, iv);
             code[q] = cw;
@@ -1277,7 +1350,7 @@ __global__ void __launch_bounds__(kThreads, (kQuery ? query_three_ctas(C::W, C::
         uint32_t hits = 0;
         const uint32_t code_mem = smem_addr(code);
         if constexpr (kQuery) {
-            if constexpr (C::W < 6 && C::M <= 8) {
+            if constexpr (C::W < 6 && C::M * C::kBits <= 16) {
                 hits = query_strip_direct<C>(code_mem, vmask, p.shard_mask, p.words);
             } else {
                 constexpr int kWarpBytes = query_warp_bytes(C::W, C::H);

@@ -89,3 +89,45 @@ def test_query_matches_oracle(sbf, cuda, oracle_mod, cfg):
             np.testing.assert_array_equal(out.cpu().numpy(), want)
             got = np.unpackbits(bits.cpu().numpy().view(np.uint8), bitorder="little")
             np.testing.assert_array_equal(got[:want.size], want)
+
+
+PROTEINS = [(12, 10, 6, 4), (12, 12, 6, 8), (12, 8, 4, 16), (12, 5, 9, 4), (7, 6, 7, 4),
+            (1, 1, 1, 4)]
+
+
+@pytest.mark.parametrize("k,s,m,h", PROTEINS)
+def test_protein_tiles_match_oracle(sbf, cuda, oracle_mod, k, s, m, h):
+    """Proteins in the kernels compiled at run time: every byte value,
+    invalid bytes at every spacing up to twice the window length, and the
+    edges of strips and tiles."""
+    torch = cuda
+    rng = np.random.default_rng(k * 100 + m)
+    seq = random_dna(rng, 20_000, b"ACDEFGHIKLMNPQRSTVWYacdefghiklmnpqrstvwy")
+    at, step = 9_000, 1
+    while at < 14_000:
+        seq[at] = rng.choice(np.frombuffer(b"*@[`{-\0\xc1", np.uint8))
+        at += step
+        step = step % (2 * k) + 1
+    seq[14_000:16_000] = rng.integers(0, 256, 2_000, dtype=np.uint8)
+    seq[17_000:17_500] = np.resize(seq[:5], 500)
+    cfg = dict(k=k, s=s, m=m, hashes=h, alphabet=sbf.ALPHABET_PROTEIN)
+    o = oracle_mod.Oracle(**cfg)
+    f = sbf.Filter(1 << 17, **cfg)
+    assert f.kernel_path() == sbf.Filter.KERNELS_RUNTIME_COMPILED
+    for n in (1, 31, 32, 33, 1023, 1025, 8191, 8192, 8193, 16_385, 19_900):
+        for shift in (0, 3):
+            part = seq[shift:][:n + k - 1]
+            words = o.new_words(1 << 17)
+            o.insert(words, part[:part.size // 2 + k])
+            f.clear()
+            f.insert_sequence_async(on_device(torch, part[:part.size // 2 + k], shift))
+            np.testing.assert_array_equal(f.words_host(), words)
+            want = o.contains(words, part)
+            d = on_device(torch, part, shift)
+            out = torch.full((want.size,), 7, dtype=torch.uint8, device="cuda")
+            f.contains_sequence_async(d, out)
+            bits = torch.full(((want.size + 31) // 32,), -1, dtype=torch.int32, device="cuda")
+            f.contains_sequence_bits_async(d, bits)
+            np.testing.assert_array_equal(out.cpu().numpy(), want)
+            got = np.unpackbits(bits.cpu().numpy().view(np.uint8), bitorder="little")
+            np.testing.assert_array_equal(got[:want.size], want)
