@@ -34,7 +34,7 @@ constexpr int kInsertSlotBytes = kFlushSlots * kThreads * 32;  // dynamic smem o
 #define SBF_SIZE_FN constexpr
 #endif
 SBF_SIZE_FN bool query_three_ctas(int w, int h) { return w >= 10 && w <= 16 && h <= 8; }
-SBF_SIZE_FN int query_pool_slots(int w, int h) { return query_three_ctas(w, h) ? 208 : 344; }
+SBF_SIZE_FN int query_pool_slots(int w, int h) { return query_three_ctas(w, h) ? 208 : 336; }
 SBF_SIZE_FN int query_warp_bytes(int w, int h) { return query_pool_slots(w, h) * (32 + 4); }
 SBF_SIZE_FN int query_cta_bytes(int w, int h) { return kThreads / 32 * query_warp_bytes(w, h); }
 
@@ -170,12 +170,15 @@ const KernelSet* generic_kernels();
 // Auxiliary kernels (sbf_kernels.cu).
 cudaError_t launch_pack_dense(const uint8_t* seq, uint64_t num_symbols, uint64_t* words,
                               cudaStream_t stream);
-// Ragged launches: tile_rec[t] = first record whose end exceeds the first
-// input byte of tile t (n_ranges when none).
-cudaError_t launch_tile_records(const DevRange* ranges, uint64_t n_ranges, int64_t sym_base,
-                                uint64_t tile_kmers, uint64_t n_tiles, uint32_t* tile_rec,
-                                cudaStream_t stream);
-// The same with the record and tile counts read from `sizes` on the device;
+// Before a ragged pass (n_tiles > 0): tile_rec[t] = first record whose end
+// exceeds the first input byte of tile t (n_ranges when none), the queue
+// counter at zero, and zero_a and zero_b (n_ranges entries each; both or
+// neither) at zero.
+cudaError_t launch_ragged_prepare(const DevRange* ranges, uint64_t n_ranges, int64_t sym_base,
+                                  uint64_t tile_kmers, uint64_t n_tiles, uint32_t* tile_rec,
+                                  unsigned int* queue, unsigned long long* zero_a,
+                                  unsigned long long* zero_b, cudaStream_t stream);
+// The tile records with the record and tile counts read from `sizes` on the device;
 // `max_tiles` bounds the launch.
 cudaError_t launch_tile_records_sized(const DevRange* ranges, const DevSizes* sizes,
                                       int64_t sym_base, uint64_t max_tiles, uint32_t* tile_rec,

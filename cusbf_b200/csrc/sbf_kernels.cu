@@ -13,40 +13,52 @@
 
 namespace sbf {
 
-// tile_rec[t] = first record whose end exceeds the first byte tile t stages
-// (binary search; records sorted and non-overlapping).
-__global__ void tile_records_kernel(const DevRange* ranges, uint64_t n, int64_t sym_base,
-                                    uint64_t tile_kmers, uint64_t n_tiles, uint32_t* tile_rec) {
-    const uint64_t t = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (t >= n_tiles) return;
-    const int64_t s0 = static_cast<int64_t>(t * tile_kmers) + sym_base;
+// First record whose end exceeds byte x (records sorted and non-overlapping).
+__device__ __forceinline__ uint32_t first_record_past(const DevRange* ranges, uint64_t n,
+                                                      int64_t x) {
     uint64_t lo = 0, hi = n;
     while (lo < hi) {
         const uint64_t mid = (lo + hi) >> 1;
-        if (static_cast<int64_t>(ranges[mid].offset + ranges[mid].bytes) > s0)
+        if (static_cast<int64_t>(ranges[mid].offset + ranges[mid].bytes) > x)
             hi = mid;
         else
             lo = mid + 1;
     }
-    tile_rec[t] = static_cast<uint32_t>(lo);
+    return static_cast<uint32_t>(lo);
+}
+
+// tile_rec[t] = first record whose end exceeds the first byte tile t stages.
+__global__ void tile_records_kernel(const DevRange* ranges, uint64_t n, int64_t sym_base,
+                                    uint64_t tile_kmers, uint64_t n_tiles, uint32_t* tile_rec) {
+    const uint64_t t = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (t < n_tiles)
+        tile_rec[t] = first_record_past(ranges, n, static_cast<int64_t>(t * tile_kmers) + sym_base);
+}
+
+// All that a ragged pass needs before its tile kernel, in one launch: the
+// tiles' first records, the queue counter at zero and, when given, the
+// per-record tallies at zero.  (As a kernel and three memsets a small ragged
+// query with counts took 17.7 us, this way 13.1.)
+__global__ void ragged_prepare_kernel(const DevRange* ranges, uint64_t n, int64_t sym_base,
+                                      uint64_t tile_kmers, uint64_t n_tiles, uint32_t* tile_rec,
+                                      unsigned int* queue, unsigned long long* zero_a,
+                                      unsigned long long* zero_b) {
+    const uint64_t first = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
+    if (first == 0) *queue = 0u;
+    for (uint64_t t = first; t < n_tiles; t += stride)
+        tile_rec[t] = first_record_past(ranges, n, static_cast<int64_t>(t * tile_kmers) + sym_base);
+    if (zero_a)
+        for (uint64_t i = first; i < n; i += stride) zero_a[i] = zero_b[i] = 0;
 }
 
 // tile_records_kernel with the record and tile counts read on the device.
 __global__ void tile_records_sized_kernel(const DevRange* ranges, const DevSizes* sizes,
                                           int64_t sym_base, uint32_t* tile_rec) {
     const uint64_t t = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (t >= sizes->n_tiles) return;
-    const uint64_t n = sizes->n_ranges;
-    const int64_t s0 = static_cast<int64_t>(t) * kTileKmers + sym_base;
-    uint64_t lo = 0, hi = n;
-    while (lo < hi) {
-        const uint64_t mid = (lo + hi) >> 1;
-        if (static_cast<int64_t>(ranges[mid].offset + ranges[mid].bytes) > s0)
-            hi = mid;
-        else
-            lo = mid + 1;
-    }
-    tile_rec[t] = static_cast<uint32_t>(lo);
+    if (t < sizes->n_tiles)
+        tile_rec[t] = first_record_past(ranges, sizes->n_ranges,
+                                        static_cast<int64_t>(t * kTileKmers) + sym_base);
 }
 
 // ---------------------------------------------------------------------------
@@ -94,12 +106,14 @@ cudaError_t launch_pack_dense(const uint8_t* seq, uint64_t num_symbols, uint64_t
 
 const void* tile_records_kernel_ptr() { return reinterpret_cast<const void*>(&tile_records_kernel); }
 
-cudaError_t launch_tile_records(const DevRange* ranges, uint64_t n_ranges, int64_t sym_base,
-                                uint64_t tile_kmers, uint64_t n_tiles, uint32_t* tile_rec,
-                                cudaStream_t stream) {
-    if (n_tiles == 0) return cudaSuccess;
-    tile_records_kernel<<<static_cast<unsigned>((n_tiles + 255) / 256), 256, 0, stream>>>(
-        ranges, n_ranges, sym_base, tile_kmers, n_tiles, tile_rec);
+cudaError_t launch_ragged_prepare(const DevRange* ranges, uint64_t n_ranges, int64_t sym_base,
+                                  uint64_t tile_kmers, uint64_t n_tiles, uint32_t* tile_rec,
+                                  unsigned int* queue, unsigned long long* zero_a,
+                                  unsigned long long* zero_b, cudaStream_t stream) {
+    const uint64_t work = zero_a && n_ranges > n_tiles ? n_ranges : n_tiles;
+    const uint64_t blocks = (work + 255) / 256;
+    ragged_prepare_kernel<<<static_cast<unsigned>(blocks < 4096 ? blocks : 4096), 256, 0, stream>>>(
+        ranges, n_ranges, sym_base, tile_kmers, n_tiles, tile_rec, queue, zero_a, zero_b);
     return cudaGetLastError();
 }
 

@@ -213,13 +213,14 @@ static unsigned ragged_grid(const sbf_filter* f, bool query, uint64_t n_tiles, u
 }
 
 int ragged_launch(sbf_filter* f, bool query, const TileParams& p, uint32_t ctas,
-                  cudaStream_t st, StripKernel kernel) {
+                  cudaStream_t st, StripKernel kernel, bool zero_tallies) {
     if (p.n_tiles == 0) return SBF_OK;
     const int which = query ? kQueryRagged : kInsertRagged;
     if (!kernel.fn) kernel = {f->ks->fn(which), kStrip};
-    SBF_CUDA(launch_tile_records(p.ranges, p.n_ranges, p.sym_base, kernel.tile_kmers(), p.n_tiles,
-                                 const_cast<uint32_t*>(p.tile_rec), st));
-    SBF_CUDA(cudaMemsetAsync(p.queue, 0, sizeof(unsigned int), st));
+    SBF_CUDA(launch_ragged_prepare(p.ranges, p.n_ranges, p.sym_base, kernel.tile_kmers(), p.n_tiles,
+                                   const_cast<uint32_t*>(p.tile_rec), p.queue,
+                                   zero_tallies ? p.rec_valid : nullptr,
+                                   zero_tallies ? p.rec_pos : nullptr, st));
     SBF_CUDA(launch_set_kernel(f->ks, kernel.fn, ragged_grid(f, query, p.n_tiles, ctas),
                                which, p, st));
     f->launches += 2;
@@ -585,12 +586,14 @@ static int ragged_async(sbf_filter_t* f, bool query, const char* d_seq, uint64_t
     if (tally && n && !d_rec_pos)
         return set_error(SBF_ERR_INVALID_ARGUMENT, "per-record count arrays are null");
     cudaStream_t st = S_(stream);
-    if (tally && n) {
-        SBF_CUDA(cudaMemsetAsync(d_rec_valid, 0, n * sizeof(uint64_t), st));
-        SBF_CUDA(cudaMemsetAsync(d_rec_pos, 0, n * sizeof(uint64_t), st));
-    }
     const uint64_t W = f->kmers_of_bytes(len);
-    if (W == 0) return SBF_OK;
+    if (W == 0) {
+        if (tally && n) {
+            SBF_CUDA(cudaMemsetAsync(d_rec_valid, 0, n * sizeof(uint64_t), st));
+            SBF_CUDA(cudaMemsetAsync(d_rec_pos, 0, n * sizeof(uint64_t), st));
+        }
+        return SBF_OK;
+    }
     if (!d_seq) return set_error(SBF_ERR_INVALID_ARGUMENT, "sequence pointer is null");
     // With per-record counts the hit bytes are optional.
     if (query && (tally ? (d_out && out_len < W) : (!d_out || out_len < W)))
@@ -614,7 +617,8 @@ static int ragged_async(sbf_filter_t* f, bool query, const char* d_seq, uint64_t
     p.n_tiles = (p.n_kmers + static_cast<uint64_t>(-p.sym_base) + tile - 1) / tile;
     SBF_TRY(r->direct_tile_rec.ensure(p.n_tiles * 4 + 64));
     p.tile_rec = static_cast<const uint32_t*>(r->direct_tile_rec.ptr);
-    return ragged_launch(f, query, p, 0, st, kernel);
+    // The launch that prepares the pass also zeroes the tallies.
+    return ragged_launch(f, query, p, 0, st, kernel, tally);
 }
 
 extern "C" int sbf_ragged_insert_async(sbf_filter_t* f, const char* d_seq, uint64_t len,

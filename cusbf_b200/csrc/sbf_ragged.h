@@ -19,10 +19,12 @@ TileParams ragged_params(const sbf_filter* f, bool query, const uint8_t* d_seq, 
                          uint8_t* d_out, unsigned int* queue, unsigned long long* counts,
                          bool out_bits = false);
 
-// Stream launch of one ragged pass: tile records, queue reset, tile kernel (the
+// Stream launch of one ragged pass: tile records, queue reset and, with
+// `zero_tallies`, p.rec_valid and p.rec_pos at zero; then the tile kernel (the
 // set's own unless `kernel` is given; p.n_tiles counts its tiles).
 int ragged_launch(sbf_filter* f, bool query, const TileParams& p, uint32_t ctas,
-                  cudaStream_t st, StripKernel kernel = {nullptr, kStrip});
+                  cudaStream_t st, StripKernel kernel = {nullptr, kStrip},
+                  bool zero_tallies = false);
 
 // The same pass replayed as a graph whose two kernel nodes are updated per
 // launch (built on first use).
