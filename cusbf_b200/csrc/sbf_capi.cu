@@ -178,8 +178,11 @@ int sbf_filter::launch(bool query, bool dense, const void* input, uint64_t input
     p.n_tiles = (n_kmers + static_cast<uint64_t>(phase) + tile - 1) / tile;
     p.err = d_err;
     p.gen = gen;
-    const uint64_t resident = static_cast<uint64_t>(sms) * static_cast<uint64_t>(occupancy[which]);
-    const uint64_t grid = std::min<uint64_t>(p.n_tiles, std::max<uint64_t>(resident, 1));
+    // A CTA per tile for the tile kernels (see tile_kernel); the generic kernels
+    // walk strips with a resident grid.
+    uint64_t grid = std::min<uint64_t>(p.n_tiles, 0x7FFFFFFFu);
+    if (!ks->is_tile(which))
+        grid = std::min<uint64_t>(grid, static_cast<uint64_t>(sms) * occupancy[which]);
     SBF_CUDA(launch_set_kernel(ks, kernel.fn, static_cast<unsigned>(grid), which, p, st));
     ++launches;
     return SBF_OK;

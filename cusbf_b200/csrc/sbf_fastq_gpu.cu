@@ -575,7 +575,7 @@ int FastqDevice::launch_block_graph(sbf_filter* f, bool query, bool fasta, const
         (s = ctl.ensure(128)) != SBF_OK || (s = grow<uint64_t>(line_end, line_cap + 1)) != SBF_OK ||
         (s = grow<DevRange>(seq, line_cap)) != SBF_OK || (s = grow<DevRange>(hdr, line_cap)) != SBF_OK ||
         (s = counts.ensure(64)) != SBF_OK || (s = g_sizes.ensure(sizeof(DevSizes))) != SBF_OK ||
-        (s = g_summary.ensure(sizeof(BlockSummary))) != SBF_OK || (s = g_queue.ensure(64)) != SBF_OK ||
+        (s = g_summary.ensure(sizeof(BlockSummary))) != SBF_OK ||
         (s = g_tile_rec.ensure(max_tiles * 4 + 64)) != SBF_OK ||
         (s = h_summary.ensure(sizeof(BlockSummary))) != SBF_OK)
         return s;
@@ -612,13 +612,11 @@ int FastqDevice::launch_block_graph(sbf_filter* f, bool query, bool fasta, const
     p.ranges = static_cast<const DevRange*>(seq.ptr);
     p.n_ranges = cap;
     p.tile_rec = static_cast<const uint32_t*>(g_tile_rec.ptr);
-    p.queue = static_cast<unsigned int*>(g_queue.ptr);
     p.counts = d_counts;
     p.gen = f->gen;
     p.sizes = d_sizes;
-    const int occ = f->occupancy[query ? 5 : 4];
-    const unsigned tile_grid = static_cast<unsigned>(std::max<uint64_t>(
-        std::min<uint64_t>(max_tiles, static_cast<uint64_t>(f->sms) * std::max(occ, 1)), 1));
+    // A CTA per possible tile: those past the device's count return at once.
+    const unsigned tile_grid = static_cast<unsigned>(std::min<uint64_t>(max_tiles, 0x7FFFFFFFu));
     const void* tile_fn = query ? f->ks->query_ragged : f->ks->insert_ragged;
 
     cudaError_t e;
@@ -665,8 +663,7 @@ int FastqDevice::launch_block_graph(sbf_filter* f, bool query, bool fasta, const
                                                 d_sum);
         }
         if ((r = launch_tile_records_sized(p.ranges, d_sizes, p.sym_base, max_tiles,
-                                           const_cast<uint32_t*>(p.tile_rec), st)) != cudaSuccess ||
-            (r = cudaMemsetAsync(p.queue, 0, sizeof(unsigned int), st)) != cudaSuccess)
+                                           const_cast<uint32_t*>(p.tile_rec), st)) != cudaSuccess)
             return r;
         TileParams copy = p;
         void* args[] = {&copy};
@@ -749,7 +746,6 @@ void FastqDevice::release() {
     line_cap = 0;
     g_sizes.release();
     g_summary.release();
-    g_queue.release();
     g_tile_rec.release();
     h_summary.release();
     line_len.release();

@@ -49,7 +49,7 @@ struct BlockSummary {
 struct FastqDevice {
     DevBuf text, tile_off, line_end, seq, hdr, ctl, counts, out, rec_counts;
     DevBuf line_len, line_hdr, comp;  // FASTA line tables and compacted sequence
-    DevBuf g_sizes, g_summary, g_queue, g_tile_rec;  // graph replay
+    DevBuf g_sizes, g_summary, g_tile_rec;  // graph replay
     PinnedBuf h_hits, h_comp, h_summary;
     // One executable per (FASTA?, query?): blocks of one kind update theirs in
     // place; a different kind never forces a re-instantiation.

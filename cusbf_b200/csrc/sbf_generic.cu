@@ -35,6 +35,9 @@ const KernelSet kGeneric = {
     generic_ptr<true, false, true>(),
     0,
     0,
+    false,
+    8,
+    true,
 };
 
 // Dense packing for any alphabet (pack_dense_sequence_kernel,

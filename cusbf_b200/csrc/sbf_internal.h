@@ -10,9 +10,9 @@
 namespace sbf {
 
 // Launch geometry of the tile kernels.
-constexpr int kThreads = 256;                          // threads per CTA
+constexpr int kThreads = 128;                          // threads per CTA
 constexpr int kStrip = 32;                             // consecutive k-mers per thread
-constexpr int kTileKmers = kThreads * kStrip;          // k-mers per tile (8192)
+constexpr int kTileKmers = kThreads * kStrip;          // k-mers per tile (4096)
 constexpr int kStripWords = 4;                         // code words one strip reads
 constexpr int kCodeWords = (kThreads - 1) * (kStrip / 16) + kStripWords;  // per tile
 constexpr int kStageBytes = kCodeWords * 16 + 64;      // staged input bytes per buffer
@@ -24,25 +24,25 @@ constexpr int kInsertSlotBytes = kFlushSlots * kThreads * 32;  // dynamic smem o
 // every slot.  A warp of random sequence needs 121 slots at W = 16 m-mers a
 // window and 171 at W = 11 (the runs of 32 strips less the borrowed ones),
 // with a deviation of 6 to 8; a warp that needs more takes several rounds.
-// Three CTAs of 256 threads and 80 registers fit an SM with 208 slots a warp;
-// shorter windows change runs more often (252 slots at W = 8) and longer ones
-// and more than eight hashes need more registers, so those run two CTAs.
+// 24 warps of 80 registers a thread fit an SM with 208 slots each; shorter
+// windows change runs more often (252 slots at W = 8) and longer ones and more
+// than eight hashes need more registers, so those run 16 warps an SM.
 // Run-time compilation takes device functions only.
 #ifdef __CUDACC_RTC__
 #define SBF_SIZE_FN __device__ constexpr
 #else
 #define SBF_SIZE_FN constexpr
 #endif
-SBF_SIZE_FN bool query_three_ctas(int w, int h) { return w >= 10 && w <= 16 && h <= 8; }
-SBF_SIZE_FN int query_pool_slots(int w, int h) { return query_three_ctas(w, h) ? 208 : 336; }
+SBF_SIZE_FN bool query_24_warps(int w, int h) { return w >= 10 && w <= 16 && h <= 8; }
+SBF_SIZE_FN int query_pool_slots(int w, int h) { return query_24_warps(w, h) ? 208 : 336; }
 SBF_SIZE_FN int query_warp_bytes(int w, int h) { return query_pool_slots(w, h) * (32 + 4); }
 SBF_SIZE_FN int query_cta_bytes(int w, int h) { return kThreads / 32 * query_warp_bytes(w, h); }
 
 // The insert kernels' part of a warp: the same pool, filled with the runs' word
 // masks, and a spare slot per lane for a run that a neighbour flushes.  184
-// slots leave room for three CTAs and 4 deviations at W = 12 (158 slots).
-SBF_SIZE_FN bool insert_three_ctas(int w, int h) { return w >= 12 && w <= 16 && h <= 8; }
-SBF_SIZE_FN int insert_pool_slots(int w, int h) { return insert_three_ctas(w, h) ? 184 : 312; }
+// slots leave room for 24 warps and 4 deviations at W = 12 (158 slots).
+SBF_SIZE_FN bool insert_24_warps(int w, int h) { return w >= 12 && w <= 16 && h <= 8; }
+SBF_SIZE_FN int insert_pool_slots(int w, int h) { return insert_24_warps(w, h) ? 184 : 304; }
 SBF_SIZE_FN int insert_warp_bytes(int w, int h) {
     return insert_pool_slots(w, h) * (32 + 4) + 32 * 32;
 }
@@ -93,7 +93,6 @@ struct TileParams {
     const DevRange* ranges;
     uint64_t n_ranges;
     const uint32_t* tile_rec;      // per tile: first record whose end > tile start
-    unsigned int* queue;           // work-queue counter, zero before the launch
     unsigned long long* counts;    // [0] valid windows, [1] positive windows
     // Optional per-record tallies (zeroed before the launch): valid and
     // positive windows of record r are added to rec_valid[r << rec_shift]
@@ -133,17 +132,20 @@ struct KernelSet {
     int smem_insert = insert_cta_bytes(k - m + 1, h);
     int smem_query = query_cta_bytes(k - m + 1, h);
     bool jit = false;    // loaded from a run-time compiled library
-    int jit_occupancy = 2;  // resident CTAs per SM assumed for run-time compiled sets
+    int jit_occupancy = 4;  // resident CTAs per SM assumed for run-time compiled sets
     const void* fn(int which) const {
         const void* const fns[6] = {insert_bytes, query_bytes,   insert_dense,
                                     query_dense,  insert_ragged, query_ragged};
         return fns[which];
     }
-    // Protein tile sets: the dense kernels are the generic ones.
-    bool generic_dense = false;
+    // Sets of generic kernels; protein tile sets have generic dense kernels.
+    bool generic = false, generic_dense = false;
+    bool is_tile(int which) const {
+        return !generic && !(generic_dense && (which == 2 || which == 3));
+    }
     int smem(int which) const {
         const bool query = (which & 1) != 0;
-        if (generic_dense && (which == 2 || which == 3)) return query ? 0 : kInsertSlotBytes;
+        if (!generic && !is_tile(which)) return query ? 0 : kInsertSlotBytes;
         return query ? smem_query : smem_insert;
     }
 };
@@ -171,13 +173,12 @@ const KernelSet* generic_kernels();
 cudaError_t launch_pack_dense(const uint8_t* seq, uint64_t num_symbols, uint64_t* words,
                               cudaStream_t stream);
 // Before a ragged pass (n_tiles > 0): tile_rec[t] = first record whose end
-// exceeds the first input byte of tile t (n_ranges when none), the queue
-// counter at zero, and zero_a and zero_b (n_ranges entries each; both or
-// neither) at zero.
+// exceeds the first input byte of tile t (n_ranges when none), and zero_a and
+// zero_b (n_ranges entries each; both or neither) at zero.
 cudaError_t launch_ragged_prepare(const DevRange* ranges, uint64_t n_ranges, int64_t sym_base,
                                   uint64_t tile_kmers, uint64_t n_tiles, uint32_t* tile_rec,
-                                  unsigned int* queue, unsigned long long* zero_a,
-                                  unsigned long long* zero_b, cudaStream_t stream);
+                                  unsigned long long* zero_a, unsigned long long* zero_b,
+                                  cudaStream_t stream);
 // The tile records with the record and tile counts read from `sizes` on the device;
 // `max_tiles` bounds the launch.
 cudaError_t launch_tile_records_sized(const DevRange* ranges, const DevSizes* sizes,

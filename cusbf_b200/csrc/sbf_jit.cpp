@@ -322,9 +322,10 @@ const KernelSet* jit_kernels(int k, int s, int m, int h, int alphabet, int devic
         } else {
             // The generic kernels use few registers; inserts take the flush
             // ring's dynamic shared memory, queries none.
+            e->ks.generic = true;
             e->ks.smem_insert = kInsertSlotBytes;
             e->ks.smem_query = 0;
-            e->ks.jit_occupancy = 4;
+            e->ks.jit_occupancy = 8;
         }
         it = g_sets.emplace(key, std::move(e)).first;
     }

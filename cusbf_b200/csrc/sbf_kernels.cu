@@ -36,16 +36,14 @@ __global__ void tile_records_kernel(const DevRange* ranges, uint64_t n, int64_t 
 }
 
 // All that a ragged pass needs before its tile kernel, in one launch: the
-// tiles' first records, the queue counter at zero and, when given, the
-// per-record tallies at zero.  (As a kernel and three memsets a small ragged
-// query with counts took 17.7 us, this way 13.1.)
+// tiles' first records and, when given, the per-record tallies at zero.  (As a
+// kernel and three memsets a small ragged query with counts took 17.7 us, this
+// way 13.1.)
 __global__ void ragged_prepare_kernel(const DevRange* ranges, uint64_t n, int64_t sym_base,
                                       uint64_t tile_kmers, uint64_t n_tiles, uint32_t* tile_rec,
-                                      unsigned int* queue, unsigned long long* zero_a,
-                                      unsigned long long* zero_b) {
+                                      unsigned long long* zero_a, unsigned long long* zero_b) {
     const uint64_t first = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-    if (first == 0) *queue = 0u;
     for (uint64_t t = first; t < n_tiles; t += stride)
         tile_rec[t] = first_record_past(ranges, n, static_cast<int64_t>(t * tile_kmers) + sym_base);
     if (zero_a)
@@ -108,12 +106,12 @@ const void* tile_records_kernel_ptr() { return reinterpret_cast<const void*>(&ti
 
 cudaError_t launch_ragged_prepare(const DevRange* ranges, uint64_t n_ranges, int64_t sym_base,
                                   uint64_t tile_kmers, uint64_t n_tiles, uint32_t* tile_rec,
-                                  unsigned int* queue, unsigned long long* zero_a,
-                                  unsigned long long* zero_b, cudaStream_t stream) {
+                                  unsigned long long* zero_a, unsigned long long* zero_b,
+                                  cudaStream_t stream) {
     const uint64_t work = zero_a && n_ranges > n_tiles ? n_ranges : n_tiles;
     const uint64_t blocks = (work + 255) / 256;
     ragged_prepare_kernel<<<static_cast<unsigned>(blocks < 4096 ? blocks : 4096), 256, 0, stream>>>(
-        ranges, n_ranges, sym_base, tile_kmers, n_tiles, tile_rec, queue, zero_a, zero_b);
+        ranges, n_ranges, sym_base, tile_kmers, n_tiles, tile_rec, zero_a, zero_b);
     return cudaGetLastError();
 }
 
@@ -183,10 +181,10 @@ const KernelSet* find_kernels(int k, int s, int m, int h) {
 //   400 k           8.3 / 6.3    8.3 / 6.3   10.3 / 8.6
 //   1.5 M          16.5 / 12.4  12.8 / 10.3  15.6 / 12.4
 //     3 M          26.4 / 20.6  22.6 / 18.5  20.6 / 16.5
-// so strips of 8 take up to two tiles an SM, strips of 16 up to three.
+// so strips of 8 take up to 16 warps an SM, strips of 16 up to 24.
 static int narrow_strip(uint64_t n_kmers, int sms) {
     const uint64_t per_sm = n_kmers / static_cast<uint64_t>(sms > 0 ? sms : 1);
-    return per_sm < 2 * 8 * kThreads ? 8 : per_sm < 3 * 16 * kThreads ? 16 : kStrip;
+    return per_sm < 16 * 32 * 8 ? 8 : per_sm < 24 * 32 * 16 ? 16 : kStrip;
 }
 
 const void* narrow16_kernel(int config, int which);

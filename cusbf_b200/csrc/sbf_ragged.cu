@@ -1,7 +1,6 @@
 // sbf_ragged.cu -- ragged batches: many records of uneven length through one
-// persistent tile-kernel launch with a device work queue, a multi-stage host
-// pipeline whose per-chunk device work can be replayed as a CUDA graph, and
-// an autotuner with a persisted table.  No reference counterpart: the
+// tile-kernel launch, a multi-stage host pipeline whose per-chunk device work
+// can be replayed as a CUDA graph, and an autotuner with a persisted table.  No reference counterpart: the
 // reference inserts a record batch by normalising it on the host (records
 // joined with one 'N', include/cusbf/normalized_record_batch.hpp:235-276)
 // and launching the plain kernel over the copy, or one launch per record
@@ -83,8 +82,7 @@ struct RaggedState {
     RaggedSlot slot[kMaxStages];
     cudaStream_t copy_stream = nullptr;  // chunk uploads
     cudaStream_t d2h_stream = nullptr;   // query result downloads
-    // [0] work-queue counter; [2..3] (as u64) batch counts.
-    unsigned int* d_ctl = nullptr;
+    unsigned int* d_ctl = nullptr;  // [2..5]: batch counts (two u64)
     DevBuf direct_tile_rec;
 };
 
@@ -175,7 +173,7 @@ static unsigned long long* ctl_counts(RaggedState* r) {
 
 TileParams ragged_params(const sbf_filter* f, bool query, const uint8_t* d_seq,
                                 uint64_t len, const DevRange* d_rng, uint64_t n,
-                                const uint32_t* d_tile_rec, uint8_t* d_out, unsigned int* queue,
+                                const uint32_t* d_tile_rec, uint8_t* d_out,
                                 unsigned long long* counts, bool out_bits) {
     TileParams p{};
     p.input = d_seq;
@@ -198,18 +196,27 @@ TileParams ragged_params(const sbf_filter* f, bool query, const uint8_t* d_seq,
     p.ranges = d_rng;
     p.n_ranges = n;
     p.tile_rec = d_tile_rec;
-    p.queue = queue;
     p.counts = counts;
     p.gen = f->gen;
     return p;
 }
 
+// CTAs of a ragged pass: four tiles each once that fills the chip (a CTA loads
+// its next tile's bytes while it works on one; with a CTA per tile the loads of
+// the tile's records were exposed: contigs 1030 us against 925, reads 2020
+// against 1940, and 1007 / 2181 with a resident grid, whose tiles the CTAs
+// share unevenly).  `ctas` limits the CTAs per SM; the generic kernels walk
+// strips with a resident grid.
 static unsigned ragged_grid(const sbf_filter* f, bool query, uint64_t n_tiles, uint32_t ctas) {
-    const int occ = f->occupancy[query ? 5 : 4];
+    const int which = query ? kQueryRagged : kInsertRagged;
+    const int occ = f->occupancy[which];
     const uint64_t per_sm = ctas == 0 ? static_cast<uint64_t>(occ)
                                       : std::min<uint64_t>(ctas, static_cast<uint64_t>(occ));
     const uint64_t resident = static_cast<uint64_t>(f->sms) * std::max<uint64_t>(per_sm, 1);
-    return static_cast<unsigned>(std::max<uint64_t>(std::min<uint64_t>(n_tiles, resident), 1));
+    uint64_t grid = std::min<uint64_t>(n_tiles, resident);
+    if (ctas == 0 && f->ks->is_tile(which))
+        grid = std::max<uint64_t>(grid, std::min<uint64_t>((n_tiles + 3) / 4, 0x7FFFFFFFu));
+    return static_cast<unsigned>(std::max<uint64_t>(grid, 1));
 }
 
 int ragged_launch(sbf_filter* f, bool query, const TileParams& p, uint32_t ctas,
@@ -218,7 +225,7 @@ int ragged_launch(sbf_filter* f, bool query, const TileParams& p, uint32_t ctas,
     const int which = query ? kQueryRagged : kInsertRagged;
     if (!kernel.fn) kernel = {f->ks->fn(which), kStrip};
     SBF_CUDA(launch_ragged_prepare(p.ranges, p.n_ranges, p.sym_base, kernel.tile_kmers(), p.n_tiles,
-                                   const_cast<uint32_t*>(p.tile_rec), p.queue,
+                                   const_cast<uint32_t*>(p.tile_rec),
                                    zero_tallies ? p.rec_valid : nullptr,
                                    zero_tallies ? p.rec_pos : nullptr, st));
     SBF_CUDA(launch_set_kernel(f->ks, kernel.fn, ragged_grid(f, query, p.n_tiles, ctas),
@@ -258,15 +265,7 @@ int ragged_graph_launch(sbf_filter* f, RaggedGraph& g, bool query, const TilePar
     if (!g.exec) {
         SBF_CUDA(cudaGraphCreate(&g.graph, 0));
         SBF_CUDA(cudaGraphAddKernelNode(&g.n_rec, g.graph, nullptr, 0, &rk));
-        cudaMemsetParams ms{};
-        ms.dst = p.queue;
-        ms.value = 0;
-        ms.elementSize = sizeof(unsigned int);
-        ms.width = 1;
-        ms.height = 1;
-        cudaGraphNode_t n_ms;
-        SBF_CUDA(cudaGraphAddMemsetNode(&n_ms, g.graph, &g.n_rec, 1, &ms));
-        SBF_CUDA(cudaGraphAddKernelNode(&g.n_tile, g.graph, &n_ms, 1, &tk));
+        SBF_CUDA(cudaGraphAddKernelNode(&g.n_tile, g.graph, &g.n_rec, 1, &tk));
         SBF_CUDA(cudaGraphInstantiate(&g.exec, g.graph, 0));
     } else {
         SBF_CUDA(cudaGraphExecKernelNodeSetParams(g.exec, g.n_rec, &rk));
@@ -502,7 +501,7 @@ static int ragged_pipeline(sbf_filter* f, bool query, const char* h_seq, uint64_
             clip_ranges_kernel<<<blocks, 256, 0, st>>>(s.d_rng, np, b_lo, b_hi);
             SBF_CUDA(cudaGetLastError());
             const TileParams p = ragged_params(f, query, s.d_seq, b_hi - b_lo, s.d_rng, np,
-                                               s.d_tile_rec, s.d_out, r->d_ctl, d_counts, kbits);
+                                               s.d_tile_rec, s.d_out, d_counts, kbits);
             if (t.use_graph)
                 SBF_TRY(ragged_graph_launch(f, s.graph[query ? 1 : 0], query, p, t.ctas_per_sm,
                                             st));
@@ -606,7 +605,6 @@ static int ragged_async(sbf_filter_t* f, bool query, const char* d_seq, uint64_t
     }
     TileParams p = ragged_params(f, query, reinterpret_cast<const uint8_t*>(d_seq), len,
                                  reinterpret_cast<const DevRange*>(d_ranges), n, nullptr, d_out,
-                                 r->d_ctl,
                                  d_counts ? reinterpret_cast<unsigned long long*>(d_counts)
                                           : ctl_counts(r));
     p.rec_valid = reinterpret_cast<unsigned long long*>(d_rec_valid);

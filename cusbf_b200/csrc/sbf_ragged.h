@@ -16,11 +16,11 @@ namespace sbf {
 // bit i % 32 of word i / 32).
 TileParams ragged_params(const sbf_filter* f, bool query, const uint8_t* d_seq, uint64_t len,
                          const DevRange* d_rng, uint64_t n, const uint32_t* d_tile_rec,
-                         uint8_t* d_out, unsigned int* queue, unsigned long long* counts,
+                         uint8_t* d_out, unsigned long long* counts,
                          bool out_bits = false);
 
-// Stream launch of one ragged pass: tile records, queue reset and, with
-// `zero_tallies`, p.rec_valid and p.rec_pos at zero; then the tile kernel (the
+// Stream launch of one ragged pass: tile records and, with `zero_tallies`,
+// p.rec_valid and p.rec_pos at zero; then the tile kernel (the
 // set's own unless `kernel` is given; p.n_tiles counts its tiles).
 int ragged_launch(sbf_filter* f, bool query, const TileParams& p, uint32_t ctas,
                   cudaStream_t st, StripKernel kernel = {nullptr, kStrip},

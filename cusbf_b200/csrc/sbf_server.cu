@@ -227,7 +227,7 @@ struct Server {
     cudaStream_t up = nullptr, comp = nullptr, down = nullptr;
     uint8_t* d_ring = nullptr;
     uint8_t* h_ring = nullptr;
-    unsigned int* d_ctl = nullptr;  // [0] work-queue counter, [2..9] counts
+    unsigned int* d_ctl = nullptr;  // [2..9]: counts
     Ring dring, hring;
     RaggedGraph graph[2];
 
@@ -577,8 +577,7 @@ int Server::launch(SrvBatch* b) {
     if (k) {
         TileParams p =
             ragged_params(f, query, d_seq, b->seq_bytes, d_rng, k, d_tile, tally ? nullptr : d_out,
-                          d_ctl, reinterpret_cast<unsigned long long*>(d_ctl + 2) + (query ? 2 : 0),
-                          bits);
+                          reinterpret_cast<unsigned long long*>(d_ctl + 2) + (query ? 2 : 0), bits);
         if (tally) {
             // (valid, positive) pairs per record, accumulated by the kernel.
             if ((e = cudaMemsetAsync(d_out, 0, k * 16, comp)) != cudaSuccess)

@@ -25,10 +25,10 @@ namespace sbf {
 namespace {
 
 // Per-CTA record staging in dynamic shared memory: kLogRecords records of a
-// 4-byte shard id and four 8-byte masks.  A tile of 8192 windows emits about
-// 1000 runs of uniform DNA; a tile with more than kLogRecords runs appends the
+// 4-byte shard id and four 8-byte masks.  A tile of 4096 windows emits about
+// 500 runs of uniform DNA; a tile with more than kLogRecords runs appends the
 // excess to the global log one record at a time.
-constexpr int kLogRecords = 1536;
+constexpr int kLogRecords = 768;
 constexpr int kEmitSmem = kLogRecords * (32 + 4);
 
 struct RunLog {
@@ -113,12 +113,12 @@ __device__ __forceinline__ void insert_strip(const uint32_t* c, uint32_t vmask,
     if (prev_valid) flush(1u, prev_shard, acc);
 }
 
-// The insert tile path (plain loads for staging) with each super-k-mer run
+// The insert tile path with each super-k-mer run
 // appended to the CTA's shared-memory log; at the end of every tile the CTA
 // reserves a contiguous range of the global log with one atomic and copies
 // its records there.
 template <class C>
-__global__ void __launch_bounds__(kThreads, 2) emit_kernel(TileParams p, RunLog log) {
+__global__ void __launch_bounds__(kThreads, 4) emit_kernel(TileParams p, RunLog log) {
     __shared__ alignas(16) uint8_t stage[kStageBytes];
     __shared__ uint32_t code[kCodeWords + 4];
     __shared__ uint32_t inval[kCodeWords + 4];
@@ -280,7 +280,7 @@ extern "C" int sbf_emit_runs_async(const sbf_filter_t* f, const char* d_seq, uin
     p.n_tiles = (n_kmers + kTileKmers - 1) / kTileKmers;
     p.err = f->d_err;
     RunLog log{d_shards, d_masks, capacity, reinterpret_cast<unsigned long long*>(d_count)};
-    const uint64_t grid = std::min<uint64_t>(p.n_tiles, static_cast<uint64_t>(f->sms) * 2);
+    const uint64_t grid = std::min<uint64_t>(p.n_tiles, static_cast<uint64_t>(f->sms) * 4);
     es->fn<<<static_cast<unsigned>(grid), kThreads, kEmitSmem, st>>>(p, log);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "emit_kernel");
     return SBF_OK;
@@ -310,7 +310,7 @@ extern "C" int sbf_apply_runs_async(sbf_filter_t* f, const uint32_t* d_shards,
         ring_set[f->device] = 1;
     }
     const uint64_t blocks = std::min<uint64_t>((n + kThreads - 1) / kThreads,
-                                               static_cast<uint64_t>(f->sms) * 2);
+                                               static_cast<uint64_t>(f->sms) * 4);
     apply_runs_kernel<<<static_cast<unsigned>(blocks), kThreads, kInsertSlotBytes, st>>>(
         d_shards, d_masks, n, f->d_words, shard_lo, shard_hi, f->d_err);
     const cudaError_t e = cudaGetLastError();

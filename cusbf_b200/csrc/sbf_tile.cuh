@@ -8,16 +8,15 @@
 // and their dense-packed twins).  Results are bit-identical to it; the work
 // decomposition is new:
 //
-//   * A persistent CTA (two or three per SM) walks tiles of 8192 consecutive
-//     windows (2048 or 4096 in small launches).  Each tile's input bytes are staged into shared memory by
-//     a 1D bulk async copy (TMA) on an mbarrier, issued as soon as the tile
-//     before it is encoded, so copies overlap hashing.  Only the 16-byte aligned
-//     interior goes through the bulk copy; ragged edges are read with plain
-//     loads, so nothing outside the caller's buffer is touched.  Every wait
-//     is bounded and reports kDevErrStageTimeout instead of hanging.
+//   * A CTA of 128 threads takes a tile of 4096 consecutive windows (1024 or
+//     2048 in small launches).  The tile's input bytes are staged into shared
+//     memory by a 1D bulk async copy (TMA) on an mbarrier.  Only the 16-byte
+//     aligned interior goes through the bulk copy; ragged edges are read with
+//     plain loads, so nothing outside the caller's buffer is touched.  Every
+//     wait is bounded and reports kDevErrStageTimeout instead of hanging.
 //   * Staged bytes are encoded with SWAR into 2-bit code words (16 bases per
 //     32-bit word, earliest base in the top bits) plus invalid masks.
-//   * Each of the 256 threads owns a strip of 32 consecutive windows (8 or
+//   * Each thread owns a strip of 32 consecutive windows (8 or
 //     16 in small launches).  Every
 //     m-mer and s-mer of the strip is a funnel shift of the code words,
 //     every position is hashed once, and the per-window minimizer is a
@@ -35,9 +34,8 @@
 //   * Insert ORs the one-hot masks of a run's s-mers in registers, stores them
 //     to the run's slot, and has the warp OR the slots into their shards, four
 //     lanes and one request each.
-//   * Ragged launches take tiles from a device work-queue counter and drop
-//     windows that cross a record boundary or touch a byte outside every
-//     record (marked per tile in shared memory).
+//   * Ragged launches drop windows that cross a record boundary or touch a byte
+//     outside every record (marked per tile in shared memory).
 #pragma once
 
 #include "sbf_device.cuh"
@@ -1105,7 +1103,7 @@ __device__ __forceinline__ void insert_strip_runs(uint32_t code_mem, uint32_t vm
 // first, first + kThreads, ... of those overlapping the tile.
 template <class C>
 __device__ __forceinline__ void mark_records(const TileParams& p, int64_t s0, uint32_t first,
-                                             uint32_t* inval, uint32_t* brk) {
+                                             DevRange rec, uint32_t* inval, uint32_t* brk) {
     constexpr int64_t kSpan = C::kSpan;
     const int64_t len = static_cast<int64_t>(p.input_bytes);
     const int64_t t_end = s0 + kSpan;
@@ -1130,7 +1128,7 @@ __device__ __forceinline__ void mark_records(const TileParams& p, int64_t s0, ui
         set_bits(inval, gap0, until);
     }
     for (uint64_t r = first + threadIdx.x; r < n; r += kThreads) {
-        const DevRange rec = p.ranges[r];
+        if (r >= first + kThreads) rec = p.ranges[r];
         const int64_t a = static_cast<int64_t>(rec.offset);
         if (a >= t_end) break;
         const int64_t b = a + static_cast<int64_t>(rec.bytes);
@@ -1224,16 +1222,18 @@ __device__ __forceinline__ void tally_records(const TileParams& p, uint32_t firs
     if (kf != kNone && lane == static_cast<uint32_t>(__ffs(grp) - 1)) add(kf, tot);
 }
 
-// Persistent tile kernel.  Plain launches walk tiles blockIdx.x + i * gridDim.x;
-// ragged launches take tiles from the device work-queue counter p.queue, so
-// tiles of uneven cost (records of any length, N runs) balance across CTAs.
-// Either way tile i+2 is taken while tile i is processed, and tile i+1's
-// staging copy is issued once tile i's bytes are encoded, into the same buffer.
+// The tile kernel.  A plain launch has a CTA per tile; a smaller grid's CTAs walk
+// tiles blockIdx.x + i * gridDim.x, each with the next tile's copy in flight.
+// Six CTAs of 128 threads an SM, with the tiles handed out by the hardware,
+// keep all 24 warps busy to the end and cost little at the barriers.  A
+// persistent grid was slower: its CTAs share an SM's issue slots unevenly, so
+// that some finish early and leave 18.5 warps on average (100 Mbp insert 488 us against 435, 10 M reads 5.95 ms
+// against 5.15; CTAs of 256 threads 452 and 5.38, of 64 threads 453 and 5.32).
 template <class C, bool kQuery, bool kDense, bool kRagged>
-__global__ void __launch_bounds__(kThreads, (kQuery ? query_three_ctas(C::W, C::H)
-                                                    : insert_three_ctas(C::W, C::H))
-                                                ? 3
-                                                : 2)
+__global__ void __launch_bounds__(kThreads, (kQuery ? query_24_warps(C::W, C::H)
+                                                    : insert_24_warps(C::W, C::H))
+                                                ? 24 * 32 / kThreads
+                                                : 16 * 32 / kThreads)
     tile_kernel(TileParams p) {
     constexpr int kCodeWords = C::kCodeWords;
     __shared__ alignas(128) uint8_t stage[C::kStageBytes];
@@ -1241,12 +1241,12 @@ __global__ void __launch_bounds__(kThreads, (kQuery ? query_three_ctas(C::W, C::
     // One bit per position: invalid bases, record starts.
     __shared__ alignas(8) uint32_t inval[C::kSpan / 32 + 2];
     __shared__ alignas(8) uint32_t brk[kRagged ? C::kSpan / 32 + 2 : 1];
-    __shared__ uint64_t tiles[3];
-    __shared__ uint32_t first_rec[3], last_rec[3];
-    __shared__ unsigned long long tally[2];
     __shared__ bool covered;  // the staged tile needs no plain loads
     __shared__ alignas(8) uint64_t bar;
     __shared__ uint64_t onehot[kQuery ? 1 : 64];
+    // Dynamic shared memory, a part per warp: the pools of query_strip and
+    // insert_strip_runs.
+    extern __shared__ __align__(16) uint64_t slots[];
 
     const int tid = threadIdx.x;
     if constexpr (!kQuery) onehot_init(onehot);
@@ -1259,45 +1259,31 @@ __global__ void __launch_bounds__(kThreads, (kQuery ? query_three_ctas(C::W, C::
             p.n_ranges = z.n_ranges;
         }
     }
-    auto take = [&](uint32_t i, int slot) {
-        uint64_t t;
-        if constexpr (kRagged) {
-            t = atomicAdd(p.queue, 1u);
-            first_rec[slot] = t < p.n_tiles ? p.tile_rec[t] : 0u;
-            last_rec[slot] =
-                t + 1 < p.n_tiles ? p.tile_rec[t + 1] : static_cast<uint32_t>(p.n_ranges);
-        } else {
-            t = blockIdx.x + static_cast<uint64_t>(i) * gridDim.x;
-        }
-        tiles[slot] = t;
-        return t;
-    };
     if (tid == 0) {
         mbar_init(&bar, 1);
         mbar_fence_init();
-        tally[0] = tally[1] = 0;
-        const uint64_t t0 = take(0, 0);
-        take(1, 1);
-        if (t0 < p.n_tiles) covered = issue_stage<C, kDense>(p, t0, stage, &bar);
+        if (blockIdx.x < p.n_tiles) covered = issue_stage<C, kDense>(p, blockIdx.x, stage, &bar);
     }
     __syncthreads();
-    // Dynamic shared memory: the query kernel's pool of shard slots, a part per
-    // warp (query_cta_bytes per CTA), or the insert kernel's flush staging ring,
-    // [slot][thread] (kInsertSlotBytes per CTA).
-    extern __shared__ __align__(16) uint64_t slots[];
     unsigned long long n_valid = 0, n_pos = 0;
     const uint32_t origin = stage_origin<C, kDense>(p);
-    for (uint32_t it = 0;; ++it) {
-        const uint64_t tile = tiles[it % 3];
-        if (tile >= p.n_tiles) break;
-        const bool ok = mbar_wait_bounded(&bar, it & 1u);
+    uint32_t parity = 0;
+    for (uint32_t tile = blockIdx.x; tile < p.n_tiles; tile += gridDim.x, parity ^= 1u) {
+        uint32_t first_rec = 0;
+        DevRange rec{0, 0};  // the thread's first record of the tile
+        if constexpr (kRagged) {
+            first_rec = p.tile_rec[tile];
+            if (first_rec + tid < p.n_ranges) rec = p.ranges[first_rec + tid];
+        }
+        const bool ok = mbar_wait_bounded(&bar, parity);
+        // (Also the barrier behind the last tile's reads of the code words.)
         if (__syncthreads_or(!ok)) {
             // The copy that ran out of time may still be in flight: give it
             // one more bounded wait before the CTA's shared memory is
             // released, so that it does not land in memory a later CTA owns.
             if (tid == 0) {
                 atomicExch(p.err, kDevErrStageTimeout);
-                (void)mbar_wait_bounded(&bar, it & 1u);
+                (void)mbar_wait_bounded(&bar, parity);
             }
             __syncthreads();
             return;
@@ -1306,7 +1292,6 @@ __global__ void __launch_bounds__(kThreads, (kQuery ? query_three_ctas(C::W, C::
             fill_ragged<kDense>(p, tile_geom<C, kDense>(p, tile), stage);
             __syncthreads();
         }
-        const int64_t s0 = tile_first_symbol<C>(p, tile);
         if constexpr (C::kBits != 2) {
             static_assert(!kDense || C::kBits == 2, "dense proteins run the generic kernels");
             for (int t = tid; t <= kThreads; t += kThreads) {
@@ -1323,17 +1308,12 @@ __global__ void __launch_bounds__(kThreads, (kQuery ? query_three_ctas(C::W, C::
         }
         if constexpr (kRagged) {
             __syncthreads();
-            mark_records<C>(p, s0, first_rec[it % 3], inval, brk);
+            mark_records<C>(p, tile_first_symbol<C>(p, tile), first_rec, rec, inval, brk);
         }
         __syncthreads();
-        if (tid == 0) {
-            // The staged bytes are encoded: the next tile's copy goes out and
-            // lands while this one is hashed.  The tile after it is taken now,
-            // so that a barrier lies between its slot's write and its reads.
-            const uint64_t next = tiles[(it + 1) % 3];
-            if (next < p.n_tiles) covered = issue_stage<C, kDense>(p, next, stage, &bar);
-            take(it + 2, (it + 2) % 3);
-        }
+        // In a limited grid the CTA's next tile lands while this one is hashed.
+        if (tid == 0 && tile + gridDim.x < p.n_tiles)
+            covered = issue_stage<C, kDense>(p, tile + gridDim.x, stage, &bar);
 
         auto strip_bits = [&](const uint32_t* a) {
             const uint32_t* w = a + (tid * C::kStrip) / 32;
@@ -1345,8 +1325,11 @@ __global__ void __launch_bounds__(kThreads, (kQuery ? query_three_ctas(C::W, C::
                        (static_cast<uint64_t>(__funnelshift_r(w[1], w[2], sh)) << 32);
             }
         };
-        const int64_t first_kmer = s0 + static_cast<int64_t>(tid) * C::kStrip;
-        uint32_t vmask = strip_valid<C>(strip_bits(inval), first_kmer, p.n_kmers);
+        // (Made again after the passes over the strip: a live copy spilled.)
+        auto first_window = [&] {
+            return tile_first_symbol<C>(p, tile) + static_cast<int64_t>(tid) * C::kStrip;
+        };
+        uint32_t vmask = strip_valid<C>(strip_bits(inval), first_window(), p.n_kmers);
         if constexpr (kRagged) {
             vmask = strip_in_record<C>(strip_bits(brk), vmask);
             n_valid += __popc(vmask);
@@ -1361,6 +1344,7 @@ __global__ void __launch_bounds__(kThreads, (kQuery ? query_three_ctas(C::W, C::
                 hits = query_strip<C>(code_mem, vmask, p.shard_mask, p.words,
                                       smem_addr(slots) + (tid >> 5) * kWarpBytes);
             }
+            const int64_t first_kmer = first_window();
             if (p.out) store_strip_bytes<C>(hits, p.out, first_kmer, p.n_kmers);
             if constexpr (kRagged) n_pos += __popc(hits & vmask);
             if (p.out_bits) store_strip_bits<C>(hits, p.out_bits, first_kmer, p.n_kmers);
@@ -1370,24 +1354,28 @@ __global__ void __launch_bounds__(kThreads, (kQuery ? query_three_ctas(C::W, C::
                                  smem_addr(slots) + (tid >> 5) * kWarpBytes, onehot);
         }
         if constexpr (kRagged) {
-            if (p.rec_valid)
-                tally_records(p, first_rec[it % 3], last_rec[it % 3], first_kmer, vmask, hits);
+            if (p.rec_valid) {
+                const uint32_t last = tile + 1 < p.n_tiles ? p.tile_rec[tile + 1]
+                                                           : static_cast<uint32_t>(p.n_ranges);
+                tally_records(p, p.tile_rec[tile], last, first_window(), vmask, hits);
+            }
         }
     }
     if constexpr (kRagged) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            n_valid += __shfl_down_sync(0xFFFFFFFFu, n_valid, o);
-            n_pos += __shfl_down_sync(0xFFFFFFFFu, n_pos, o);
-        }
+        // A warp sees at most 2^31 windows of a launch.
+        const uint32_t valid = __reduce_add_sync(0xFFFFFFFFu, static_cast<uint32_t>(n_valid));
+        const uint32_t pos = __reduce_add_sync(0xFFFFFFFFu, static_cast<uint32_t>(n_pos));
+        __shared__ uint32_t tally[kThreads / 32][2];
         if ((tid & 31) == 0) {
-            atomicAdd(&tally[0], n_valid);
-            atomicAdd(&tally[1], n_pos);
+            tally[tid >> 5][0] = valid;
+            tally[tid >> 5][1] = pos;
         }
         __syncthreads();
-        if (tid == 0) {
-            atomicAdd(p.counts, tally[0]);
-            atomicAdd(p.counts + 1, tally[1]);
+        if (tid < 2) {
+            unsigned long long sum = 0;
+#pragma unroll
+            for (int w = 0; w < kThreads / 32; ++w) sum += tally[w][tid];
+            if (sum) atomicAdd(p.counts + tid, sum);
         }
     }
 }

@@ -359,8 +359,7 @@ int sbf_record_batch_counts_noalloc(const sbf_filter_t* filter, const char* d_se
 /* ---- Ragged batches (no reference counterpart) ------------------------
  *
  * Many records of uneven length in one buffer, processed in place by one
- * persistent kernel launch whose CTAs take tiles from a device work queue.
- * Records are (offset, bytes) ranges into the buffer, sorted by offset and
+ * tile-kernel launch.  Records are (offset, bytes) ranges into the buffer, sorted by offset and
  * non-overlapping (gaps allowed).  Exactly the windows that lie inside one
  * record are inserted / queried: the result equals one insert_sequence /
  * contains_sequence per record (filter.cuh:154-190, :464-533), the

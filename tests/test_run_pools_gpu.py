@@ -1,6 +1,6 @@
 """The tile kernels' run lists and slot pools against the oracle, where a pool
 takes one round, several rounds or none, and at the edges of strips, warps and
-tiles (2048, 4096 and 8192 windows for strips of 8, 16 and 32 windows, which
+tiles (1024, 2048 and 4096 windows for strips of 8, 16 and 32 windows, which
 the launch size selects: on 148 SMs up to 606,207 and 1,818,623 windows)."""
 import numpy as np
 import pytest
@@ -22,7 +22,7 @@ CONFIGS = [
 ]
 
 
-LENGTHS = (1, 7, 8, 9, 31, 32, 33, 255, 256, 257, 2047, 2048, 2049, 60_000, 819_199, 819_200,
+LENGTHS = (1, 7, 8, 9, 31, 32, 33, 255, 256, 257, 1023, 1024, 1025, 60_000, 819_199, 819_200,
            819_201, 1_884_159, 1_884_160, 1_884_161)
 IDS = ["-".join(map(str, c.values())) for c in CONFIGS]
 
