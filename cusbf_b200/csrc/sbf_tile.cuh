@@ -16,11 +16,10 @@
 //     wait is bounded and reports kDevErrStageTimeout instead of hanging.
 //   * Staged bytes are encoded with SWAR into 2-bit code words (16 bases per
 //     32-bit word, earliest base in the top bits) plus invalid masks.
-//   * Each thread owns a strip of 32 consecutive windows (8 or
-//     16 in small launches).  Every
-//     m-mer and s-mer of the strip is a funnel shift of the code words,
-//     every position is hashed once, and the per-window minimizer is a
-//     Gil-Werman sliding minimum over blocks of W positions (about 3
+//   * Each thread owns a strip of 32 consecutive windows (8 or 16 in small
+//     launches).  Every m-mer and s-mer of the strip is a funnel shift of the
+//     code words, every position is hashed once, and the per-window minimizer
+//     is a Gil-Werman sliding minimum over blocks of W positions (about 3
 //     comparisons per window, one more for W > 16, where the reference hashes
 //     and compares all W m-mers of every window).
 //   * Both list a strip's super-k-mer runs (consecutive windows that select
@@ -209,8 +208,8 @@ __device__ __forceinline__ void encode_word(uint32_t origin, const uint8_t* buf,
 // Encodes the 32 protein symbols from grid position 32 t into five code words
 // (5 bits a symbol, earliest symbol in the top bits) and a word of invalid
 // bits.  Letters only, either case; code = letter - 'A'.  With the rest of the
-// tile kernel as for DNA, 64 M residues of <12,10,6,4> take 287 us to query and
-// 362 to insert, where a byte load and a whole window's hashes per window took
+// tile kernel as for DNA, 64 M residues of <12,10,6,4> take 260 us to query and
+// 302 to insert, where a byte load and a whole window's hashes per window took
 // 647 and 736 (sbf_generic.cuh).
 __device__ __forceinline__ void encode_protein_strip(uint32_t origin, const uint8_t* buf, int t,
                                                      uint32_t* code, uint32_t* inval) {
@@ -369,8 +368,9 @@ __device__ __forceinline__ uint32_t strip_valid(uint64_t bits, int64_t first_kme
 // word gets one bit: the first word's mask is read from `onehot` (1 << b for
 // b = 0..63 in the CTA's shared memory) and the others are 64-bit shifts.
 // The table spares the logic pipe two instructions a word, but 32 random
-// entries take about six passes of the shared-memory pipe: 100 Mbp took 531
-// us with four loads, 494 with three or two, 488 with one and 494 with none.
+// entries take about six passes of the shared-memory pipe: 100 Mbp plain and
+// 200 Mbp of contigs take 429 and 936 us with two loads, 433 and 924 with one,
+// 100 Mbp 444 with none.
 template <class C>
 __device__ __forceinline__ void smer_masks(const uint32_t* c, int r, uint64_t m[4],
                                            const uint64_t* onehot) {
@@ -549,6 +549,23 @@ __device__ __forceinline__ void copy_u32_if(uint32_t pred, uint32_t dst, uint32_
         : "memory");
 }
 
+// The shard ids of a lane's slots, from its run list: head b's entry is the
+// number of runs that start up to it.  Four heads a turn (the busiest lane of
+// a warp has about 7): a 4 Mbp query took 19.8 us, with one head a turn 20.4.
+__device__ __forceinline__ void list_shard_ids(uint32_t heads, uint32_t chg, uint32_t list,
+                                               uint32_t ids) {
+    while (__any_sync(0xFFFFFFFFu, heads != 0u)) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const uint32_t b = heads & (0u - heads);
+            heads ^= b;
+            const uint32_t e = __popc(chg & (b ^ (b - 1u)));
+            copy_u32_if(b, ids + 4 * u, list - 128 + 128 * e);
+        }
+        ids += 16;
+    }
+}
+
 // Copies the shards of slots e = lane / 2, lane / 2 + 16, ... below `total`
 // into the pool, a lane pair per slot: its two 16-byte copies go out in one
 // instruction and make one 32-byte request (a lane that issued both made two,
@@ -576,7 +593,6 @@ __device__ __forceinline__ void copy_shards(uint32_t total, uint32_t pool, uint3
     }
     cp_async_commit();
 }
-
 
 // Findere test of the window's F s-mers (F = 3 or 4) with byte permutes.  A bit
 // address is a byte n (upper three bits) and a bit t in it: for each shard
@@ -761,14 +777,16 @@ __device__ __noinline__ uint3 list_runs(uint32_t code_mem, uint32_t list) {
 // that lane's last run continues into the strip.  Lanes whose runs do not fit
 // the pool any more wait for another round.
 //
-// Bound: the integer logic pipe (72% busy on <31,28,16,4>), then the latency
-// of the shard copies.  1.51e9 positions of 10 M reads against 8 GiB: 5.95 ms,
-// 25 G shards/s; with the copies issued by the thread that finds a run (two
+// Bound: the integer logic pipe (on <31,28,16,4> about 55 of its instructions
+// per window, which alone take 4.5 of the 5.11 ms), then the latency of the
+// shard copies.  1.51e9 positions of 10 M reads against 8 GiB: 5.11 ms, 29 G
+// shards/s; with the copies issued by the thread that finds a run (two
 // requests per shard), a copy slot per thread and shifts for the bit tests it
 // was 7.82 ms at 19 G shards/s, the rate at which the memory takes two 16-byte
 // requests each.  Loading the shards to registers instead keeps the L1 lines
-// of all requests in flight and was slower with every byte of shared memory
-// in use (6.8 ms at 150 KB an SM, 8.6 at 203 KB).
+// of all requests in flight and was slower the more shared memory the CTAs
+// hold (6.8 ms at 150 KB an SM, 8.6 at 203 KB, before the CTAs had 128
+// threads).
 template <class C>
 __device__ __forceinline__ uint32_t query_strip(uint32_t code_mem, uint32_t vmask,
                                                 uint32_t shard_mask, const uint64_t* words,
@@ -807,12 +825,7 @@ __device__ __forceinline__ uint32_t query_strip(uint32_t code_mem, uint32_t vmas
         // number of runs that start up to it.
         const uint32_t ids = run_mem + 32 * kPoolSlots;
         uint32_t rest = borrow ? heads & (heads - 1u) : heads;
-        for (uint32_t at = ids + 4 * begin; __any_sync(0xFFFFFFFFu, rest != 0u); at += 4) {
-            const uint32_t b = rest & (0u - rest);
-            rest ^= b;
-            const uint32_t e = __popc(chg & (b ^ (b - 1u))) - 1;
-            copy_u32_if(b, at, list + 128 * e);
-        }
+        list_shard_ids(rest, chg, list, ids + 4 * begin);
         __syncwarp();
         copy_shards(__reduce_max_sync(0xFFFFFFFFu, fits ? end : 0u), run_mem, ids, shard_mask,
                     words);
@@ -857,10 +870,11 @@ __device__ __forceinline__ uint32_t query_strip(uint32_t code_mem, uint32_t vmas
 }
 
 // Query of one strip without a pool: each run head loads its shard when it is
-// reached.  For windows of less than 6 m-mers of at most 8 bases, whose runs are so short (a head
-// every second window at W = 3) that a pool would take several rounds, and
-// whose m-mers are so few that the shards stay in the caches: 100 M windows of
-// <5,4,3,4> took 0.32 ms, two rounds through the pool 1.53.
+// reached.  For windows of less than 6 m-mers of at most 8 bases, whose runs
+// are so short (a head every second window at W = 3) that a pool would take
+// several rounds, and whose m-mers are so few that the shards stay in the
+// caches: 100 M windows of <5,4,3,4> took 0.32 ms, two rounds through the pool
+// 1.53.
 template <class C>
 __device__ __forceinline__ uint32_t query_strip_direct(uint32_t code_mem, uint32_t vmask,
                                                        uint32_t shard_mask,
@@ -976,11 +990,12 @@ __device__ __forceinline__ void flush_pool(uint32_t total, uint32_t pool, uint32
 // flushes the slots.
 //
 // Bound: the memory's rate of random read-modify-writes for filters beyond L2
-// (20 G shards/s at 8 GiB, 31 at 256 MiB), else the integer logic pipe.  3.1
-// Gbp into 8 GiB 18.4 ms and 100 Mbp into 256 MiB 488 us; with each window
-// issuing the flush of a run that ends there (a predicated 32-byte bulk
-// reduction, strips flushing the runs between them twice) it was 21.1 ms and
-// 688 us.
+// (20 G shards/s at 8 GiB, 31 at 256 MiB; a genome's repeats raise that by
+// what L2 holds of them), else the integer logic pipe.  3.1 Gbp into 8 GiB
+// 15.8 ms (23 G runs/s) and 100 Mbp into 256 MiB 433 us (27 G runs/s); with
+// each window issuing the flush of a run that ends there (a predicated 32-byte
+// bulk reduction, strips flushing the runs between them twice) it was 21.1 ms
+// and 688 us.
 template <class C>
 __device__ __forceinline__ void insert_strip_runs(uint32_t code_mem, uint32_t vmask,
                                                   uint32_t shard_mask, uint64_t* words,
@@ -1158,9 +1173,10 @@ __device__ __forceinline__ uint32_t strip_in_record(uint64_t bits, uint32_t vmas
 // window, between the first records of the tile and of the next one: five
 // dependent loads for reads, where all of 2 M records took 21 and a sixth of
 // the query's time, 2.46 against 2.01 ms) and a walk over the record ends;
-// empty records are skipped by the walk.  Across the warp, the record a strip starts in is usually the one the
-// previous strip ended in: a strip's last record is handed to the next lane
-// when it is that lane's first, and lanes holding the same record are summed
+// empty records are skipped by the walk.  Across the warp, the record a strip
+// starts in is usually the one the previous strip ended in: a strip's last
+// record is handed to the next lane when it is that lane's first, and lanes
+// holding the same record are summed
 // with one match + reduce, so a warp issues about one atomic pair per record
 // it touches (count_positive_kmers_per_record_kernel,
 // detail/count_positive_kmers.cuh:21-45, fused into the query epilogue).
@@ -1222,13 +1238,14 @@ __device__ __forceinline__ void tally_records(const TileParams& p, uint32_t firs
     if (kf != kNone && lane == static_cast<uint32_t>(__ffs(grp) - 1)) add(kf, tot);
 }
 
-// The tile kernel.  A plain launch has a CTA per tile; a smaller grid's CTAs walk
-// tiles blockIdx.x + i * gridDim.x, each with the next tile's copy in flight.
-// Six CTAs of 128 threads an SM, with the tiles handed out by the hardware,
-// keep all 24 warps busy to the end and cost little at the barriers.  A
-// persistent grid was slower: its CTAs share an SM's issue slots unevenly, so
-// that some finish early and leave 18.5 warps on average (100 Mbp insert 488 us against 435, 10 M reads 5.95 ms
-// against 5.15; CTAs of 256 threads 452 and 5.38, of 64 threads 453 and 5.32).
+// The tile kernel.  A plain launch has a CTA per tile; a smaller grid's CTAs
+// walk tiles blockIdx.x + i * gridDim.x, each with the next tile's copy in
+// flight.  Six CTAs of 128 threads an SM, with the tiles handed out by the
+// hardware, keep all 24 warps busy to the end and cost little at the barriers.
+// A persistent grid was slower: its CTAs share an SM's issue slots unevenly,
+// so that some finish early and leave 18.5 warps on average (100 Mbp insert
+// 488 us against 433, 10 M reads 5.95 ms against 5.12; with a CTA per tile of
+// 256 threads 452 and 5.38, of 64 threads 453 and 5.32).
 template <class C, bool kQuery, bool kDense, bool kRagged>
 __global__ void __launch_bounds__(kThreads, (kQuery ? query_24_warps(C::W, C::H)
                                                     : insert_24_warps(C::W, C::H))
