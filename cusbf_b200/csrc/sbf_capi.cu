@@ -178,11 +178,10 @@ int sbf_filter::launch(bool query, bool dense, const void* input, uint64_t input
     p.n_tiles = (n_kmers + static_cast<uint64_t>(phase) + tile - 1) / tile;
     p.err = d_err;
     p.gen = gen;
-    // A CTA per tile for the tile kernels (see tile_kernel); the generic kernels
-    // walk strips with a resident grid.
-    uint64_t grid = std::min<uint64_t>(p.n_tiles, 0x7FFFFFFFu);
-    if (!ks->is_tile(which))
-        grid = std::min<uint64_t>(grid, static_cast<uint64_t>(sms) * occupancy[which]);
+    // A CTA per tile (see tile_kernel).  The generic kernels' strips too: 64 M
+    // residues of dense <12,10,6,4> take 620 us to query and 772 to insert, with
+    // a resident grid 705 and 817; of plain <8,6,8,4> 594 and 1030, 612 and 1112.
+    const uint64_t grid = std::min<uint64_t>(p.n_tiles, 0x7FFFFFFFu);
     SBF_CUDA(launch_set_kernel(ks, kernel.fn, static_cast<unsigned>(grid), which, p, st));
     ++launches;
     return SBF_OK;
@@ -418,10 +417,9 @@ extern "C" int sbf_filter_create(uint32_t k, uint32_t s, uint32_t m, uint32_t ha
                               ks->query_dense, ks->insert_ragged, ks->query_ragged};
         // Run-time compiled kernels have their attributes set when loaded.
         // Their occupancy is the loaded kernel's own (registers and shared
-        // memory): a persistent grid larger than what fits the SMs at once
-        // runs its last CTAs as a second wave.  When the handle does not
-        // answer, the set's assumption (two CTAs per SM for the tile
-        // kernels, as their shared memory allows) stands.
+        // memory): a resident grid larger than what fits the SMs at once runs
+        // its last CTAs as a second wave.  When the handle does not answer,
+        // the set's assumption, no more than the shared memory allows, stands.
         for (int i = 0; i < 6 && ks->jit; ++i) {
             const int dyn = ks->smem(i);
             int occ = 0;
@@ -434,7 +432,7 @@ extern "C" int sbf_filter_create(uint32_t k, uint32_t s, uint32_t m, uint32_t ha
             f->occupancy[i] = occ;
         }
         for (int i = 0; i < 6 && rc == SBF_OK && !ks->jit; ++i) {
-            // Query kernels: shard slots; insert kernels: flush staging ring.
+            // The tile kernels' run pools; the generic insert's flush ring.
             const int dyn = ks->smem(i);
             if (dyn) {
                 e = cudaFuncSetAttribute(reinterpret_cast<const void*>(fns[i]),

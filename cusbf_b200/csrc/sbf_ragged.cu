@@ -205,8 +205,9 @@ TileParams ragged_params(const sbf_filter* f, bool query, const uint8_t* d_seq,
 // its next tile's bytes while it works on one; with a CTA per tile the loads of
 // the tile's records were exposed: contigs 1030 us against 925, reads 2020
 // against 1940, and 1007 / 2181 with a resident grid, whose tiles the CTAs
-// share unevenly).  `ctas` limits the CTAs per SM; the generic kernels walk
-// strips with a resident grid.
+// share unevenly).  The generic kernels load nothing ahead and take a CTA per
+// tile (64 M residues of <8,6,8,4>: insert 1285 us, with four tiles a CTA 1388,
+// with a resident grid 1485).  `ctas` limits the CTAs per SM.
 static unsigned ragged_grid(const sbf_filter* f, bool query, uint64_t n_tiles, uint32_t ctas) {
     const int which = query ? kQueryRagged : kInsertRagged;
     const int occ = f->occupancy[which];
@@ -214,8 +215,10 @@ static unsigned ragged_grid(const sbf_filter* f, bool query, uint64_t n_tiles, u
                                       : std::min<uint64_t>(ctas, static_cast<uint64_t>(occ));
     const uint64_t resident = static_cast<uint64_t>(f->sms) * std::max<uint64_t>(per_sm, 1);
     uint64_t grid = std::min<uint64_t>(n_tiles, resident);
-    if (ctas == 0 && f->ks->is_tile(which))
-        grid = std::max<uint64_t>(grid, std::min<uint64_t>((n_tiles + 3) / 4, 0x7FFFFFFFu));
+    const uint64_t tiles_each = f->ks->is_tile(which) ? 4 : 1;
+    if (ctas == 0)
+        grid = std::max<uint64_t>(
+            grid, std::min<uint64_t>((n_tiles + tiles_each - 1) / tiles_each, 0x7FFFFFFFu));
     return static_cast<unsigned>(std::max<uint64_t>(grid, 1));
 }
 
