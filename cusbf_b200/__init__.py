@@ -748,7 +748,7 @@ _sharded_methods()
 
 
 def _ragged_methods():
-    """Ragged batches: records processed in place by one persistent launch
+    """Ragged batches: records processed in place by one launch
     (sbf_ragged_*; no reference counterpart).  Query output has one byte per
     window of the whole buffer; record r's hits are
     out[offset_r : offset_r + bytes_r - k + 1]."""

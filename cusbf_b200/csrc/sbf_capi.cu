@@ -416,10 +416,10 @@ extern "C" int sbf_filter_create(uint32_t k, uint32_t s, uint32_t m, uint32_t ha
         const void* fns[6] = {ks->insert_bytes, ks->query_bytes, ks->insert_dense,
                               ks->query_dense, ks->insert_ragged, ks->query_ragged};
         // Run-time compiled kernels have their attributes set when loaded.
-        // Their occupancy is the loaded kernel's own (registers and shared
-        // memory): a resident grid larger than what fits the SMs at once runs
-        // its last CTAs as a second wave.  When the handle does not answer,
-        // the set's assumption, no more than the shared memory allows, stands.
+        // Their occupancy (the grid of a ragged pass whose CTAs per SM are
+        // limited) is the loaded kernel's own.  When the handle does not
+        // answer, the set's assumption, no more than the shared memory
+        // allows, stands.
         for (int i = 0; i < 6 && ks->jit; ++i) {
             const int dyn = ks->smem(i);
             int occ = 0;

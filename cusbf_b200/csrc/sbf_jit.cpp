@@ -148,7 +148,7 @@ struct JitConfig {
     // configuration's but the dense ones and those with windows of less than 4
     // m-mers, whose pools take several rounds (64 M windows of <8,6,8,4>, one
     // m-mer: query 1.05 ms in the tile kernel, 0.61 in the generic one;
-    // <12,10,6,4>, seven: 0.29 and 0.65).
+    // <12,10,9,4>, four: 0.47 and 0.60; <12,10,6,4>, seven: 0.26 and 0.65).
     bool tile(int v) const {
         return alphabet == SBF_ALPHABET_DNA ||
                (alphabet == SBF_ALPHABET_PROTEIN && !kVariants[v][1] && k - m >= 3);

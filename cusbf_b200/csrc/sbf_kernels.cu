@@ -177,10 +177,11 @@ const KernelSet* find_kernels(int k, int s, int m, int h) {
 // strip; shorter strips cost more work per window (W - 1 m-mers and F - 1
 // s-mers beyond its windows) but spread over more of the chip.  <31,28,16,4>
 // insert / query with strips of 8, 16 and 32 windows, in us:
-//    30 k windows   6.7 / 5.0    7.3 / 6.3   10.3 / 8.3
-//   400 k           8.3 / 6.3    8.3 / 6.3   10.3 / 8.6
-//   1.5 M          16.5 / 12.4  12.8 / 10.3  15.6 / 12.4
-//     3 M          26.4 / 20.6  22.6 / 18.5  20.6 / 16.5
+//    30 k windows   5.2 / 4.7    6.2 / 6.2    8.3 / 6.7
+//   400 k           6.3 / 6.2    8.3 / 6.2    8.3 / 8.3
+//   800 k          10.3 / 8.3    8.3 / 8.3   10.3 / 8.3
+//   1.5 M          14.4 / 12.4  12.4 / 10.3  12.4 / 10.3 (<21,19,11,4> 12.4 / 12.4)
+//     3 M          22.6 / 19.5  18.5 / 15.4  18.5 / 14.4
 // so strips of 8 take up to 16 warps an SM, strips of 16 up to 24.
 static int narrow_strip(uint64_t n_kmers, int sms) {
     const uint64_t per_sm = n_kmers / static_cast<uint64_t>(sms > 0 ? sms : 1);
