@@ -992,7 +992,7 @@ __device__ __forceinline__ void flush_pool(uint32_t total, uint32_t pool, uint32
 // Bound: the memory's rate of random read-modify-writes for filters beyond L2
 // (20 G shards/s at 8 GiB, 31 at 256 MiB; a genome's repeats raise that by
 // what L2 holds of them), else the integer logic pipe.  3.1 Gbp into 8 GiB
-// 15.8 ms (23 G runs/s) and 100 Mbp into 256 MiB 433 us (27 G runs/s); with
+// 15.8-16.3 ms (23 G runs/s) and 100 Mbp into 256 MiB 433 us (27 G runs/s); with
 // each window issuing the flush of a run that ends there (a predicated 32-byte
 // bulk reduction, strips flushing the runs between them twice) it was 21.1 ms
 // and 688 us.
