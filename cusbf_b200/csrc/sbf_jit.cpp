@@ -9,7 +9,8 @@
 //
 // Compilation takes about ten seconds, so the cubin is cached on disk under
 // $SBF_JIT_CACHE (default ~/.cache/sbf_b200), keyed by the configuration, the
-// device architecture, the NVRTC version and a hash of the embedded source.
+// device architecture, the NVRTC version and a hash of the embedded source and
+// of the kernels that are compiled from it.
 // Proteins get the tile kernels as well (JitConfig::tile); DNA triplets and
 // dense proteins get the generic kernels (sbf_generic.cuh) compiled the same
 // way with the configuration as template constants.  SBF_JIT=0 turns this off; then, and on any failure, the filter
@@ -168,25 +169,57 @@ std::string name_expr(const JitConfig& c, int v) {
     return buf;
 }
 
-bool compile(const JitConfig& c, const std::string& arch, Compiled* out) {
+// What is compiled: the embedded headers, a source text that includes some of
+// them, the six kernels' name expressions and the options.
+const char* const kHeaders[] = {kJitInternal, kJitDevice, kJitFlush, kJitTile, kJitGeneric};
+const char* const kHeaderNames[] = {"sbf_internal.h", "sbf_device.cuh", "sbf_flush.cuh",
+                                    "sbf_tile.cuh", "sbf_generic.cuh"};
+
+struct Program {
+    std::string src;
+    std::vector<std::string> exprs;  // KernelSet order
+    std::vector<std::string> opts;
+};
+
+Program program_of(const JitConfig& c, const std::string& arch) {
+    Program p;
+    p.src = std::string(kPrelude) + (c.tile(0) ? "#include \"sbf_tile.cuh\"\n" : "") +
+            (c.tile(2) ? "" : "#include \"sbf_generic.cuh\"\n");
+    for (int v = 0; v < 6; ++v) p.exprs.push_back(name_expr(c, v));
+    p.opts = {"-arch=" + arch, "-std=c++17", "-lineinfo"};
+    return p;
+}
+
+// Cache file of a configuration: everything the cubin is made from and the
+// NVRTC version make the hash.  A host launch chooses grid, block and shared
+// memory by the kernels that program_of names, so a file compiled for others
+// must never load in their place.
+std::string cache_file(const JitConfig& c, const Program& p, int nv_major, int nv_minor) {
+    uint64_t hash = 0xcbf29ce484222325ULL;
+    auto add = [&](const char* s, size_t n) { hash = fnv1a(fnv1a(hash, s, n), "", 1); };
+    for (const char* h : kHeaders) add(h, std::strlen(h));
+    add(p.src.data(), p.src.size());
+    for (const std::string& e : p.exprs) add(e.data(), e.size());
+    for (const std::string& o : p.opts) add(o.data(), o.size());
+    const int meta[] = {c.k, c.s, c.m, c.h, c.alphabet, nv_major, nv_minor};
+    hash = fnv1a(hash, meta, sizeof meta);
+    char file[128];
+    std::snprintf(file, sizeof file, "%s_k%d_s%d_m%d_h%d_a%d_%016llx.bin",
+                  c.tile(0) ? "tile" : "generic", c.k, c.s, c.m, c.h, c.alphabet,
+                  static_cast<unsigned long long>(hash));
+    return file;
+}
+
+bool compile(const Program& p, Compiled* out) {
     const Nvrtc& nv = nvrtc();
     if (!nv.ok) return false;
-    const char* headers[] = {kJitInternal, kJitDevice, kJitFlush, kJitTile, kJitGeneric};
-    const char* names[] = {"sbf_internal.h", "sbf_device.cuh", "sbf_flush.cuh", "sbf_tile.cuh",
-                           "sbf_generic.cuh"};
-    const std::string src = std::string(kPrelude) + (c.tile(0) ? "#include \"sbf_tile.cuh\"\n" : "") +
-                            (c.tile(2) ? "" : "#include \"sbf_generic.cuh\"\n");
     nvrtcProgram prog;
-    if (nv.create(&prog, src.c_str(), "sbf_jit.cu", 5, headers, names) != NVRTC_SUCCESS)
+    if (nv.create(&prog, p.src.c_str(), "sbf_jit.cu", 5, kHeaders, kHeaderNames) != NVRTC_SUCCESS)
         return false;
-    std::vector<std::string> exprs;
-    for (int v = 0; v < 6; ++v) {
-        exprs.push_back(name_expr(c, v));
-        nv.add_name(prog, exprs.back().c_str());
-    }
-    const std::string arch_opt = "-arch=" + arch;
-    const char* opts[] = {arch_opt.c_str(), "-std=c++17", "-lineinfo"};
-    bool ok = nv.compile(prog, 3, opts) == NVRTC_SUCCESS;
+    for (const std::string& e : p.exprs) nv.add_name(prog, e.c_str());
+    std::vector<const char*> opts;
+    for (const std::string& o : p.opts) opts.push_back(o.c_str());
+    bool ok = nv.compile(prog, static_cast<int>(opts.size()), opts.data()) == NVRTC_SUCCESS;
     if (!ok && std::getenv("SBF_JIT_LOG")) {
         size_t n = 0;
         nv.log_size(prog, &n);
@@ -202,7 +235,7 @@ bool compile(const JitConfig& c, const std::string& arch, Compiled* out) {
     }
     for (int v = 0; ok && v < 6; ++v) {
         const char* lowered = nullptr;
-        ok = nv.lowered(prog, exprs[v].c_str(), &lowered) == NVRTC_SUCCESS && lowered;
+        ok = nv.lowered(prog, p.exprs[v].c_str(), &lowered) == NVRTC_SUCCESS && lowered;
         if (ok) out->names.push_back(lowered);
     }
     nv.destroy(&prog);
@@ -273,25 +306,15 @@ const KernelSet* jit_kernels(int k, int s, int m, int h, int alphabet, int devic
     if (g_failed.count(key)) return nullptr;
     auto it = g_sets.find(key);
     if (it == g_sets.end()) {
-        const std::string arch = "sm_100a";
+        const Program program = program_of(jc, "sm_100a");
         int nv_major = 0, nv_minor = 0;
         if (nvrtc().ok) nvrtc().version(&nv_major, &nv_minor);
-        uint64_t hash = 0xcbf29ce484222325ULL;
-        for (const char* src : {kJitInternal, kJitDevice, kJitFlush, kJitTile, kJitGeneric, kPrelude})
-            hash = fnv1a(hash, src, std::strlen(src));
-        const int meta[] = {k, s, m, h, alphabet, nv_major, nv_minor};
-        hash = fnv1a(hash, meta, sizeof meta);
-        hash = fnv1a(hash, arch.data(), arch.size());
-        char file[128];
-        std::snprintf(file, sizeof file, "%s_k%d_s%d_m%d_h%d_a%d_%016llx.bin",
-                      jc.tile(0) ? "tile" : "generic", k, s, m, h, alphabet,
-                      static_cast<unsigned long long>(hash));
         const std::string dir = cache_dir();
-        const std::string path = dir + "/" + file;
+        const std::string path = dir + "/" + cache_file(jc, program, nv_major, nv_minor);
         Compiled c;
         if (!read_cache(path, &c)) {
             c = Compiled{};
-            if (!compile(jc, arch, &c)) {
+            if (!compile(program, &c)) {
                 g_failed.insert(key);
                 return nullptr;
             }
