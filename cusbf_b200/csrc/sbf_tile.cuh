@@ -746,17 +746,18 @@ struct FindereTest<C, 1> {
     using type = ShiftTest<C::F>;
 };
 
-// The minimizer pass of a strip: lists its runs (one low hash word per run)
-// from shared address `list` on.  Returns the windows that start a run
-// (x) and the low hash words of window 0 and window 31 (y, z).  A function of
-// its own, so that its registers (two 64-bit arrays of W) do not add to the
-// kernel's.
-template <class C>
-__device__ __noinline__ uint3 list_runs(uint32_t code_mem, uint32_t list) {
+// The minimizer pass of a strip: lists its runs (one low hash word per run, of
+// which kFew keeps the shard id) from shared address `list` on.  Returns the
+// windows that start a run (x) and the words of the first and the last window
+// (y, z).  A function of its own, so that its registers (two 64-bit arrays of
+// W) do not add to the kernel's.
+template <class C, bool kFew>
+__device__ __noinline__ uint3 list_runs(uint32_t code_mem, uint32_t list, uint32_t shard_mask) {
     uint32_t c[C::kStripWords];
     load_code_words<C>(code_mem, c);
     uint32_t at = list, chg = 1u, first = 0, prev = 0;
     for_each_min<C>(c, [&](int j, uint32_t lo) {
+        if constexpr (kFew) lo &= shard_mask;
         if (j == 0) {
             asm volatile("st.shared.u32 [%0], %1;" ::"r"(at), "r"(lo) : "memory");
             at += 128;
@@ -767,6 +768,20 @@ __device__ __noinline__ uint3 list_runs(uint32_t code_mem, uint32_t list) {
         prev = lo;
     });
     return make_uint3(chg, first, prev);
+}
+
+// The runs of a strip.  Windows with different low hash words seldom share a
+// shard unless the filter has few; then every run is one more update or copy of
+// the same 32 bytes, one after the other, so runs are told apart by shard id.
+// 100 Mbp into one shard: 1.61 ms, by hash words 6.08 (17.2 with W = 5); into
+// 16 shards 2.88, 3.08.  In larger filters the mask would cost an instruction
+// a window (4 Mbp query 20.4 us against 19.9).  Small launches mask always: one
+// pass fewer in the instruction cache (one gene 4.9 us, with both 5.5).
+template <class C>
+__device__ __forceinline__ uint3 strip_runs(uint32_t code_mem, uint32_t list,
+                                            uint32_t shard_mask) {
+    if (C::kStrip < 32 || shard_mask < 16u) return list_runs<C, true>(code_mem, list, shard_mask);
+    return list_runs<C, false>(code_mem, list, shard_mask);
 }
 
 // Query of one strip: the minimizer pass lists the strip's runs, the runs that
@@ -798,7 +813,7 @@ __device__ __forceinline__ uint32_t query_strip(uint32_t code_mem, uint32_t vmas
     uint32_t result = 0;
     while (__any_sync(0xFFFFFFFFu, vmask != 0u)) {
         const uint32_t list = run_mem + 4 * lane;
-        const uint3 runs = list_runs<C>(code_mem, list);
+        const uint3 runs = strip_runs<C>(code_mem, list, shard_mask);
         const uint32_t chg = runs.x, first = runs.y, prev = runs.z;
         // Run heads: a valid window whose predecessor is invalid or of another run.
         uint32_t heads = vmask & (chg | ~(vmask << 1));
@@ -1008,7 +1023,7 @@ __device__ __forceinline__ void insert_strip_runs(uint32_t code_mem, uint32_t vm
     const uint32_t spare = ids + 4 * kPoolSlots + 32 * lane;
     while (__any_sync(0xFFFFFFFFu, vmask != 0u)) {
         const uint32_t list = run_mem + 4 * lane;
-        const uint3 runs = list_runs<C>(code_mem, list);
+        const uint3 runs = strip_runs<C>(code_mem, list, shard_mask);
         const uint32_t chg = runs.x;
         uint32_t heads = vmask & (chg | ~(vmask << 1));
         const int n = __popc(heads);
