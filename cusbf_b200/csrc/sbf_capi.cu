@@ -173,7 +173,7 @@ int sbf_filter::launch(bool query, bool dense, const void* input, uint64_t input
     p.out = out_bits ? nullptr : out;
     p.out_bits = out_bits;
     const int which = (query ? 1 : 0) + (dense ? 2 : 0);
-    const StripKernel kernel = strip_kernel(ks, which, n_kmers, device, sms);
+    const StripKernel kernel = strip_kernel(ks, which, n_kmers, sms);
     const uint64_t tile = kernel.tile_kmers();
     p.n_tiles = (n_kmers + static_cast<uint64_t>(phase) + tile - 1) / tile;
     p.err = d_err;
@@ -449,6 +449,8 @@ extern "C" int sbf_filter_create(uint32_t k, uint32_t s, uint32_t m, uint32_t ha
             if (f->occupancy[i] < 1) f->occupancy[i] = 1;
         }
         if (rc != SBF_OK) break;
+        e = prepare_strip_kernels(ks);
+        if (e != cudaSuccess) { rc = cuda_fail(e, "cudaFuncSetAttribute(strip kernels)"); break; }
         e = cudaMalloc(&f->d_words, shards * 32);
         if (e != cudaSuccess) {
             rc = e == cudaErrorMemoryAllocation

@@ -161,7 +161,12 @@ struct StripKernel {
 };
 // The kernel of a launch of `n_kmers` windows: a set's own, or one with
 // narrower strips when the launch is small.
-StripKernel strip_kernel(const KernelSet* ks, int which, uint64_t n_kmers, int device, int sms);
+StripKernel strip_kernel(const KernelSet* ks, int which, uint64_t n_kmers, int sms);
+// Loads a set's kernels with narrower strips on the current device and lets
+// them use their dynamic shared memory.  At filter creation: a small call that
+// loaded its kernel took 4 ms, which none takes now, in a stream capture or
+// out of one.
+cudaError_t prepare_strip_kernels(const KernelSet* ks);
 
 // Returns the kernel table for a configuration, or nullptr when it is not
 // compiled into this library.

@@ -3,7 +3,6 @@
 // run time by sbf_jit.cpp) and the auxiliary kernels.
 #include <cuda_runtime.h>
 
-#include <atomic>
 #include <cstdint>
 
 #include "sbf_configs.h"
@@ -191,25 +190,30 @@ static int narrow_strip(uint64_t n_kmers, int sms) {
 const void* narrow16_kernel(int config, int which);
 const void* narrow8_kernel(int config, int which);
 
-StripKernel strip_kernel(const KernelSet* ks, int which, uint64_t n_kmers, int device, int sms) {
-    const StripKernel own{ks->fn(which), kStrip};
-    const int strip = narrow_strip(n_kmers, sms);
+// Index of a compiled set, kNumSets of any other.
+static int config_of(const KernelSet* ks) {
     int config = 0;
     while (config < kNumSets && ks != &kSets[config]) ++config;
-    if (strip == kStrip || config == kNumSets || device < 0 || device >= 64) return own;
-    const void* fn = strip == 16 ? narrow16_kernel(config, which) : narrow8_kernel(config, which);
-    // Devices on which the kernel may use its dynamic shared memory.
-    static std::atomic<uint64_t> ready[kNumSets][2][6];
-    std::atomic<uint64_t>& devices = ready[config][strip == 16][which];
-    if (!(devices.load(std::memory_order_acquire) >> device & 1u)) {
-        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 ks->smem(which)) != cudaSuccess) {
-            cudaGetLastError();
-            return own;
+    return config;
+}
+
+StripKernel strip_kernel(const KernelSet* ks, int which, uint64_t n_kmers, int sms) {
+    const int strip = narrow_strip(n_kmers, sms);
+    const int config = config_of(ks);
+    if (strip == kStrip || config == kNumSets) return {ks->fn(which), kStrip};
+    return {strip == 16 ? narrow16_kernel(config, which) : narrow8_kernel(config, which), strip};
+}
+
+cudaError_t prepare_strip_kernels(const KernelSet* ks) {
+    const int config = config_of(ks);
+    for (int which = 0; which < 6 && config < kNumSets; ++which) {
+        for (const void* fn : {narrow16_kernel(config, which), narrow8_kernel(config, which)}) {
+            const cudaError_t e = cudaFuncSetAttribute(
+                fn, cudaFuncAttributeMaxDynamicSharedMemorySize, ks->smem(which));
+            if (e != cudaSuccess) return e;
         }
-        devices.fetch_or(uint64_t{1} << device, std::memory_order_release);
     }
-    return {fn, strip};
+    return cudaSuccess;
 }
 
 cudaError_t launch_set_kernel(const KernelSet* ks, const void* fn, unsigned grid, int which,

@@ -613,7 +613,7 @@ static int ragged_async(sbf_filter_t* f, bool query, const char* d_seq, uint64_t
     p.rec_valid = reinterpret_cast<unsigned long long*>(d_rec_valid);
     p.rec_pos = reinterpret_cast<unsigned long long*>(d_rec_pos);
     const StripKernel kernel = strip_kernel(f->ks, query ? kQueryRagged : kInsertRagged, p.n_kmers,
-                                            f->device, f->sms);
+                                            f->sms);
     const uint64_t tile = kernel.tile_kmers();
     p.n_tiles = (p.n_kmers + static_cast<uint64_t>(-p.sym_base) + tile - 1) / tile;
     SBF_TRY(r->direct_tile_rec.ensure(p.n_tiles * 4 + 64));
