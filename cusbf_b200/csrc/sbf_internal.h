@@ -150,6 +150,14 @@ struct KernelSet {
     }
 };
 
+// Resident CTAs per SM of a pass that a tuning limits to `limit` units of 256
+// threads (sbf_ragged_tuning::ctas_per_sm; tuning tables hold it), 0 for no
+// limit, when `occupancy` CTAs of `threads` fit.
+inline uint64_t limited_ctas(uint32_t limit, uint32_t occupancy, uint32_t threads) {
+    const uint64_t ctas = limit ? uint64_t{limit} * 256 / threads : occupancy;
+    return ctas < 1 ? 1 : ctas < occupancy ? ctas : occupancy;
+}
+
 // Which of a set's kernels: insert or query of bytes, dense words, records.
 enum { kInsertBytes, kQueryBytes, kInsertDense, kQueryDense, kInsertRagged, kQueryRagged };
 

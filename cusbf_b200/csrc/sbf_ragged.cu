@@ -207,13 +207,12 @@ TileParams ragged_params(const sbf_filter* f, bool query, const uint8_t* d_seq,
 // against 1940, and 1007 / 2181 with a resident grid, whose tiles the CTAs
 // share unevenly).  The generic kernels load nothing ahead and take a CTA per
 // tile (64 M residues of <8,6,8,4>: insert 1285 us, with four tiles a CTA 1388,
-// with a resident grid 1485).  `ctas` limits the CTAs per SM.
+// with a resident grid 1485).  `ctas` limits the warps per SM (limited_ctas).
 static unsigned ragged_grid(const sbf_filter* f, bool query, uint64_t n_tiles, uint32_t ctas) {
     const int which = query ? kQueryRagged : kInsertRagged;
-    const int occ = f->occupancy[which];
-    const uint64_t per_sm = ctas == 0 ? static_cast<uint64_t>(occ)
-                                      : std::min<uint64_t>(ctas, static_cast<uint64_t>(occ));
-    const uint64_t resident = static_cast<uint64_t>(f->sms) * std::max<uint64_t>(per_sm, 1);
+    const uint64_t resident =
+        static_cast<uint64_t>(f->sms) *
+        limited_ctas(ctas, static_cast<uint32_t>(f->occupancy[which]), kThreads);
     uint64_t grid = std::min<uint64_t>(n_tiles, resident);
     const uint64_t tiles_each = f->ks->is_tile(which) ? 4 : 1;
     if (ctas == 0)
@@ -797,8 +796,8 @@ extern "C" int sbf_ragged_autotune(sbf_filter_t* f, int query, const char* h_seq
                 }
             }
     }
-    // Warps per SM for the winner: one CTA (8 warps) instead of the
-    // occupancy limit, which leaves SM room for concurrent work.
+    // Warps per SM for the winner: 8 instead of the occupancy limit, which
+    // leaves SM room for concurrent work.
     {
         sbf_ragged_tuning t = best;
         t.ctas_per_sm = 1;

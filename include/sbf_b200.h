@@ -376,7 +376,8 @@ typedef struct {
     uint64_t chunk_bytes; /* bytes staged per chunk (default 64 MiB insert, 256 MiB
                              query; min 4096) */
     uint32_t stages;      /* chunks in flight, 1..4 (default 2 insert, 3 query) */
-    uint32_t ctas_per_sm; /* resident CTAs per SM, 0 = occupancy limit */
+    uint32_t ctas_per_sm; /* limit on the resident warps per SM, in units of 8 warps
+                             (256 threads, whatever a CTA has); 0 = occupancy limit */
     uint32_t use_graph;   /* replay each chunk's device work as a CUDA graph */
 } sbf_ragged_tuning;
 
