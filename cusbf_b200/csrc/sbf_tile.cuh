@@ -66,6 +66,11 @@ struct Cfg {
     // The passes over a strip's windows take them in turns of at most 16.
     static constexpr int kTurn = kStrip < 16 ? kStrip : 16;
     static constexpr int kTurns = kStrip / kTurn;
+    static constexpr uint32_t kAll = 0xFFFFFFFFu >> (32 - kStrip);  // a strip's windows
+    // The windows of a strip that go through the warp's pool at a time: with one
+    // or two m-mers a window, a run every 1 or 1.5 windows, strips overflow it.
+    static constexpr int kPart = W <= 2 && kBits == 2 ? 8 : kStrip;
+    static constexpr int kParts = kStrip / kPart;
     static_assert(kStrip == 8 || kStrip == 16 || kStrip == 32, "strips of 8, 16 or 32 windows");
     static_assert(kTileKmers / 4 % 16 == 0, "tiles start at one phase of 16 bytes");
     static_assert(kBits == 2 || (kBits == 5 && kStrip == 32), "DNA, or proteins in full strips");
@@ -355,9 +360,8 @@ template <class C>
 __device__ __forceinline__ uint32_t strip_valid(uint64_t bits, int64_t first_kmer,
                                                 uint64_t n_kmers) {
     constexpr int kStrip = C::kStrip;
-    constexpr uint32_t kAll = 0xFFFFFFFFu >> (32 - kStrip);
-    uint32_t vmask = kAll;
-    if (bits) vmask = ~static_cast<uint32_t>(any_in_span<C::K>(bits)) & kAll;
+    uint32_t vmask = C::kAll;
+    if (bits) vmask = ~static_cast<uint32_t>(any_in_span<C::K>(bits)) & C::kAll;
     const int64_t left = static_cast<int64_t>(n_kmers) - first_kmer;  // windows from the first on
     if (first_kmer < 0) vmask = first_kmer > -kStrip ? vmask & (~0u << -first_kmer) : 0u;
     if (left < kStrip) vmask = left > 0 ? vmask & ((1u << left) - 1u) : 0u;
@@ -470,27 +474,27 @@ __device__ __forceinline__ void next_slot_if(uint32_t pred, uint32_t& addr, uint
         : "r"(pred));
 }
 
-// The thread's strip of the tile's code words at shared address `code`: the
-// strip's first base comes to the top of c[0].
+// Strip `strip` of the tile's code words at shared address `code`: the strip's
+// first base comes to the top of c[0].
 template <class C>
-__device__ __forceinline__ void load_code_words(uint32_t code, uint32_t (&c)[C::kStripWords]) {
-    const uint32_t tid = threadIdx.x;
+__device__ __forceinline__ void load_code_words(uint32_t code, uint32_t strip,
+                                                uint32_t (&c)[C::kStripWords]) {
     if constexpr (C::kBits != 2) {
 #pragma unroll
         for (int q = 0; q < C::kStripWords; ++q)
             asm volatile("ld.shared.u32 %0, [%1];"
                          : "=r"(c[q])
-                         : "r"(code + (C::kStrip * C::kBits / 8) * tid + 4 * q)
+                         : "r"(code + (C::kStrip * C::kBits / 8) * strip + 4 * q)
                          : "memory");
     } else if constexpr (C::kStrip == 32) {
         asm volatile(
             "ld.shared.v2.u32 {%0, %1}, [%4];\n\tld.shared.v2.u32 {%2, %3}, [%4+8];"
             : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
-            : "r"(code + 8 * tid)
+            : "r"(code + 8 * strip)
             : "memory");
     } else {
         // 46 bases (16 windows of 31) are in three words.
-        const uint32_t at = code + (tid * C::kStrip / 16) * 4;
+        const uint32_t at = code + (strip * C::kStrip / 16) * 4;
         asm volatile(
             "ld.shared.u32 %0, [%3];\n\tld.shared.u32 %1, [%3+4];\n\tld.shared.u32 %2, [%3+8];"
             : "=r"(c[0]), "=r"(c[1]), "=r"(c[2])
@@ -498,7 +502,7 @@ __device__ __forceinline__ void load_code_words(uint32_t code, uint32_t (&c)[C::
             : "memory");
         c[3] = 0;
         if constexpr (C::kStrip == 8) {
-            const uint32_t sh = 16 * (tid & 1u);
+            const uint32_t sh = 16 * (strip & 1u);
             c[0] = __funnelshift_l(c[1], c[0], sh);
             c[1] = __funnelshift_l(c[2], c[1], sh);
             c[2] <<= sh;
@@ -752,9 +756,10 @@ struct FindereTest<C, 1> {
 // (y, z).  A function of its own, so that its registers (two 64-bit arrays of
 // W) do not add to the kernel's.
 template <class C, bool kFew>
-__device__ __noinline__ uint3 list_runs(uint32_t code_mem, uint32_t list, uint32_t shard_mask) {
+__device__ __noinline__ uint3 list_runs(uint32_t code_mem, uint32_t strip, uint32_t list,
+                                        uint32_t shard_mask) {
     uint32_t c[C::kStripWords];
-    load_code_words<C>(code_mem, c);
+    load_code_words<C>(code_mem, strip, c);
     uint32_t at = list, chg = 1u, first = 0, prev = 0;
     for_each_min<C>(c, [&](int j, uint32_t lo) {
         if constexpr (kFew) lo &= shard_mask;
@@ -778,10 +783,11 @@ __device__ __noinline__ uint3 list_runs(uint32_t code_mem, uint32_t list, uint32
 // a window (4 Mbp query 20.4 us against 19.9).  Small launches mask always: one
 // pass fewer in the instruction cache (one gene 4.9 us, with both 5.5).
 template <class C>
-__device__ __forceinline__ uint3 strip_runs(uint32_t code_mem, uint32_t list,
+__device__ __forceinline__ uint3 strip_runs(uint32_t code_mem, uint32_t strip, uint32_t list,
                                             uint32_t shard_mask) {
-    if (C::kStrip < 32 || shard_mask < 16u) return list_runs<C, true>(code_mem, list, shard_mask);
-    return list_runs<C, false>(code_mem, list, shard_mask);
+    if (C::kStrip < 32 || shard_mask < 16u)
+        return list_runs<C, true>(code_mem, strip, list, shard_mask);
+    return list_runs<C, false>(code_mem, strip, list, shard_mask);
 }
 
 // Query of one strip: the minimizer pass lists the strip's runs, the runs that
@@ -803,9 +809,9 @@ __device__ __forceinline__ uint3 strip_runs(uint32_t code_mem, uint32_t list,
 // hold (6.8 ms at 150 KB an SM, 8.6 at 203 KB, before the CTAs had 128
 // threads).
 template <class C>
-__device__ __forceinline__ uint32_t query_strip(uint32_t code_mem, uint32_t vmask,
-                                                uint32_t shard_mask, const uint64_t* words,
-                                                uint32_t run_mem) {
+__device__ __forceinline__ uint32_t query_strip(uint32_t code_mem, uint32_t strip,
+                                                uint32_t vmask, uint32_t shard_mask,
+                                                const uint64_t* words, uint32_t run_mem) {
     constexpr int F = C::F;
     constexpr uint32_t kPoolSlots = query_pool_slots(C::W, C::H);
     static_assert(kPoolSlots * 32 >= 32 * 128, "the run lists fit the pool");
@@ -813,7 +819,7 @@ __device__ __forceinline__ uint32_t query_strip(uint32_t code_mem, uint32_t vmas
     uint32_t result = 0;
     while (__any_sync(0xFFFFFFFFu, vmask != 0u)) {
         const uint32_t list = run_mem + 4 * lane;
-        const uint3 runs = strip_runs<C>(code_mem, list, shard_mask);
+        const uint3 runs = strip_runs<C>(code_mem, strip, list, shard_mask);
         const uint32_t chg = runs.x, first = runs.y, prev = runs.z;
         // Run heads: a valid window whose predecessor is invalid or of another run.
         uint32_t heads = vmask & (chg | ~(vmask << 1));
@@ -845,7 +851,7 @@ __device__ __forceinline__ uint32_t query_strip(uint32_t code_mem, uint32_t vmas
         copy_shards(__reduce_max_sync(0xFFFFFFFFu, fits ? end : 0u), run_mem, ids, shard_mask,
                     words);
         uint32_t c[C::kStripWords];
-        load_code_words<C>(code_mem, c);
+        load_code_words<C>(code_mem, strip, c);
         typename FindereTest<C>::type test;
 #pragma unroll
         for (int o = 0; o < F - 1; ++o) test.enter(o, smer_hash(smer_at<C>(c, o)));
@@ -884,19 +890,47 @@ __device__ __forceinline__ uint32_t query_strip(uint32_t code_mem, uint32_t vmas
     return result;
 }
 
+// Query of the thread's strip, in parts that fit the pool (Cfg::kPart): as a
+// whole it took up to four rounds, each of which goes over the minimizers and
+// the windows again.  100 Mbp in 2 MiB, windows of two m-mers (<31,28,30,4>):
+// query 0.63 ms, in rounds 0.99; insert 0.77, 1.39.  Of one (<31,28,31,4>):
+// insert 1.40, 1.96; query in 256 MiB 1.35, 1.57.  A filter of one shard has one
+// run a strip, which parts would only cut up.
+template <class C>
+__device__ __forceinline__ uint32_t query_parts(uint32_t code_mem, uint32_t vmask,
+                                                uint32_t shard_mask, const uint64_t* words,
+                                                uint32_t run_mem) {
+    if constexpr (C::kParts > 1) {
+        if (shard_mask != 0u) {
+            using Part = Cfg<C::K, C::S, C::M, C::H, C::kPart, C::kBits>;
+            uint32_t result = 0;
+#pragma unroll 1
+            for (int i = 0; i < C::kParts; ++i)
+                result |= query_strip<Part>(code_mem, threadIdx.x * C::kParts + i,
+                                            (vmask >> (i * C::kPart)) & Part::kAll, shard_mask,
+                                            words, run_mem)
+                          << (i * C::kPart);
+            return result;
+        }
+    }
+    return query_strip<C>(code_mem, threadIdx.x, vmask, shard_mask, words, run_mem);
+}
+
 // Query of one strip without a pool: each run head loads its shard when it is
 // reached.  For windows of less than 6 m-mers of at most 8 bases, whose runs
 // are so short (a head every second window at W = 3) that a pool would take
 // several rounds, and whose m-mers are so few that the shards stay in the
 // caches: 100 M windows of <5,4,3,4> took 0.32 ms, two rounds through the pool
-// 1.53.
+// 1.53.  For windows of one m-mer as well while the L2 holds the filter: 100 M
+// windows of <31,28,31,4> take 0.75 ms up to 32 MiB (1.29 through the pool in
+// parts), at 64 MiB 1.74 (1.26).
 template <class C>
-__device__ __forceinline__ uint32_t query_strip_direct(uint32_t code_mem, uint32_t vmask,
-                                                       uint32_t shard_mask,
+__device__ __forceinline__ uint32_t query_strip_direct(uint32_t code_mem, uint32_t strip,
+                                                       uint32_t vmask, uint32_t shard_mask,
                                                        const uint64_t* words) {
     constexpr int F = C::F;
     uint32_t c[C::kStripWords];
-    load_code_words<C>(code_mem, c);
+    load_code_words<C>(code_mem, strip, c);
     typename FindereTest<C>::type test;
 #pragma unroll
     for (int o = 0; o < F - 1; ++o) test.enter(o, smer_hash(smer_at<C>(c, o)));
@@ -1012,9 +1046,10 @@ __device__ __forceinline__ void flush_pool(uint32_t total, uint32_t pool, uint32
 // bulk reduction, strips flushing the runs between them twice) it was 21.1 ms
 // and 688 us.
 template <class C>
-__device__ __forceinline__ void insert_strip_runs(uint32_t code_mem, uint32_t vmask,
-                                                  uint32_t shard_mask, uint64_t* words,
-                                                  uint32_t run_mem, const uint64_t* onehot) {
+__device__ __forceinline__ void insert_strip_runs(uint32_t code_mem, uint32_t strip,
+                                                  uint32_t vmask, uint32_t shard_mask,
+                                                  uint64_t* words, uint32_t run_mem,
+                                                  const uint64_t* onehot) {
     constexpr int F = C::F;
     constexpr uint32_t kPoolSlots = insert_pool_slots(C::W, C::H);
     static_assert(kPoolSlots * 32 >= 32 * 128, "the run lists fit the pool");
@@ -1023,7 +1058,7 @@ __device__ __forceinline__ void insert_strip_runs(uint32_t code_mem, uint32_t vm
     const uint32_t spare = ids + 4 * kPoolSlots + 32 * lane;
     while (__any_sync(0xFFFFFFFFu, vmask != 0u)) {
         const uint32_t list = run_mem + 4 * lane;
-        const uint3 runs = strip_runs<C>(code_mem, list, shard_mask);
+        const uint3 runs = strip_runs<C>(code_mem, strip, list, shard_mask);
         const uint32_t chg = runs.x;
         uint32_t heads = vmask & (chg | ~(vmask << 1));
         const int n = __popc(heads);
@@ -1056,7 +1091,7 @@ __device__ __forceinline__ void insert_strip_runs(uint32_t code_mem, uint32_t vm
         }
         __syncwarp();
         uint32_t c[C::kStripWords];
-        load_code_words<C>(code_mem, c);
+        load_code_words<C>(code_mem, strip, c);
         uint32_t ring[F][8];
         auto enter = [&](int r) {
             uint64_t m[4];
@@ -1120,6 +1155,25 @@ __device__ __forceinline__ void insert_strip_runs(uint32_t code_mem, uint32_t vm
         __syncwarp();  // the slots are read before another round's lists replace them
         if (fits) vmask = 0;
     }
+}
+
+// Insert of the thread's strip, in parts as in a query.
+template <class C>
+__device__ __forceinline__ void insert_parts(uint32_t code_mem, uint32_t vmask,
+                                             uint32_t shard_mask, uint64_t* words,
+                                             uint32_t run_mem, const uint64_t* onehot) {
+    if constexpr (C::kParts > 1) {
+        if (shard_mask != 0u) {
+            using Part = Cfg<C::K, C::S, C::M, C::H, C::kPart, C::kBits>;
+#pragma unroll 1
+            for (int i = 0; i < C::kParts; ++i)
+                insert_strip_runs<Part>(code_mem, threadIdx.x * C::kParts + i,
+                                        (vmask >> (i * C::kPart)) & Part::kAll, shard_mask, words,
+                                        run_mem, onehot);
+            return;
+        }
+    }
+    insert_strip_runs<C>(code_mem, threadIdx.x, vmask, shard_mask, words, run_mem, onehot);
 }
 
 // ---------------------------------------------------------------------------
@@ -1370,10 +1424,12 @@ __global__ void __launch_bounds__(kThreads, (kQuery ? query_24_warps(C::W, C::H)
         const uint32_t code_mem = smem_addr(code);
         if constexpr (kQuery) {
             if constexpr (C::W < 6 && C::M * C::kBits <= 16) {
-                hits = query_strip_direct<C>(code_mem, vmask, p.shard_mask, p.words);
+                hits = query_strip_direct<C>(code_mem, tid, vmask, p.shard_mask, p.words);
+            } else if (C::W == 1 && p.shard_mask < (32u << 20) / 32) {
+                hits = query_strip_direct<C>(code_mem, tid, vmask, p.shard_mask, p.words);
             } else {
                 constexpr int kWarpBytes = query_warp_bytes(C::W, C::H);
-                hits = query_strip<C>(code_mem, vmask, p.shard_mask, p.words,
+                hits = query_parts<C>(code_mem, vmask, p.shard_mask, p.words,
                                       smem_addr(slots) + (tid >> 5) * kWarpBytes);
             }
             const int64_t first_kmer = first_window();
@@ -1382,8 +1438,8 @@ __global__ void __launch_bounds__(kThreads, (kQuery ? query_24_warps(C::W, C::H)
             if (p.out_bits) store_strip_bits<C>(hits, p.out_bits, first_kmer, p.n_kmers);
         } else {
             constexpr int kWarpBytes = insert_warp_bytes(C::W, C::H);
-            insert_strip_runs<C>(code_mem, vmask, p.shard_mask, p.words,
-                                 smem_addr(slots) + (tid >> 5) * kWarpBytes, onehot);
+            insert_parts<C>(code_mem, vmask, p.shard_mask, p.words,
+                            smem_addr(slots) + (tid >> 5) * kWarpBytes, onehot);
         }
         if constexpr (kRagged) {
             if (p.rec_valid) {
