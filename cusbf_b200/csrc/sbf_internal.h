@@ -19,34 +19,64 @@ constexpr int kStageBytes = kCodeWords * 16 + 64;      // staged input bytes per
 constexpr int kFlushSlots = 8;                         // insert bulk-reduce staging slots
 constexpr int kInsertSlotBytes = kFlushSlots * kThreads * 32;  // dynamic smem of flush rings
 
-// A warp's dynamic shared memory in the query kernels: a pool of shard slots
-// (first the run lists of its lanes, 32 entries each) and the shard id of
-// every slot.  A warp of random sequence needs 121 slots at W = 16 m-mers a
-// window and 171 at W = 11 (the runs of 32 strips less the borrowed ones),
-// with a deviation of 6 to 8; a warp that needs more takes several rounds.
-// 24 warps of 80 registers a thread fit an SM with 208 slots each; shorter
-// windows change runs more often (252 slots at W = 8) and longer ones and more
-// than eight hashes need more registers, so those run 16 warps an SM.
 // Run-time compilation takes device functions only.
 #ifdef __CUDACC_RTC__
 #define SBF_SIZE_FN __device__ constexpr
 #else
 #define SBF_SIZE_FN constexpr
 #endif
-SBF_SIZE_FN bool query_24_warps(int w, int h) { return w >= 10 && w <= 16 && h <= 8; }
-SBF_SIZE_FN int query_pool_slots(int w, int h) { return query_24_warps(w, h) ? 208 : 336; }
-SBF_SIZE_FN int query_warp_bytes(int w, int h) { return query_pool_slots(w, h) * (32 + 4); }
-SBF_SIZE_FN int query_cta_bytes(int w, int h) { return kThreads / 32 * query_warp_bytes(w, h); }
+
+// Warps per SM that a tile kernel's registers are limited for: 24 (80 a
+// thread), 16 (128) or 8 (255).  `w` m-mers and `f` s-mers a window, `h` hashes.
+// The ring of a window's s-mers is held in registers, f entries of 8 in an
+// insert and of 2 (h = 4, f <= 8: 4) in a query, and spills when they do not
+// fit.  100 Mbp into 256 MiB, W = 16, in us with 24 / 16 / 8 warps:
+//   insert h = 4   f = 5 483 / 515    7 571 / 569   10 1136 / 643 / 711
+//                  f = 14 3227 / 771 / -    17 4633 / 1850 / 928
+//          h = 8   f = 5 659 / 660   10 1174 / 841 / 882
+//   query  h = 4   f = 7 517 / 538    8 605 / 576   10 714 / 653 / 773
+//                  f = 17 1491 / 928 / 1039    20 2304 / 1308 / 1196
+//          h = 8   f = 5 668 / 694    6 867 / 763   10 1712 / 1068 / 1232
+//                  f = 13 2720 / 1757 / 1497
+// Shorter windows change runs more often and need larger pools, longer ones
+// and more than eight hashes more registers.
+SBF_SIZE_FN int query_warps(int w, int h, int f) {
+    return f > (h <= 4 ? 18 : 11)                              ? 8
+           : w >= 10 && w <= 16 && h <= 8 && f <= (h <= 4 ? 7 : 5) ? 24
+                                                               : 16;
+}
+SBF_SIZE_FN int insert_warps(int w, int h, int f) {
+    return f > 15 ? 8 : w >= 12 && w <= 16 && h <= 8 && f <= 5 ? 24 : 16;
+}
+
+// A warp's dynamic shared memory in the query kernels: a pool of shard slots
+// (first the run lists of its lanes, 32 entries each) and the shard id of
+// every slot.  A warp of random sequence needs 121 slots at W = 16 m-mers a
+// window and 171 at W = 11 (the runs of 32 strips less the borrowed ones),
+// with a deviation of 6 to 8; a warp that needs more takes several rounds.
+// 24 warps fit an SM with 208 slots each; W = 8 needs 252.
+SBF_SIZE_FN int query_pool_slots(int w, int h, int f) {
+    return query_warps(w, h, f) == 24 ? 208 : 336;
+}
+SBF_SIZE_FN int query_warp_bytes(int w, int h, int f) {
+    return query_pool_slots(w, h, f) * (32 + 4);
+}
+SBF_SIZE_FN int query_cta_bytes(int w, int h, int f) {
+    return kThreads / 32 * query_warp_bytes(w, h, f);
+}
 
 // The insert kernels' part of a warp: the same pool, filled with the runs' word
 // masks, and a spare slot per lane for a run that a neighbour flushes.  184
 // slots leave room for 24 warps and 4 deviations at W = 12 (158 slots).
-SBF_SIZE_FN bool insert_24_warps(int w, int h) { return w >= 12 && w <= 16 && h <= 8; }
-SBF_SIZE_FN int insert_pool_slots(int w, int h) { return insert_24_warps(w, h) ? 184 : 304; }
-SBF_SIZE_FN int insert_warp_bytes(int w, int h) {
-    return insert_pool_slots(w, h) * (32 + 4) + 32 * 32;
+SBF_SIZE_FN int insert_pool_slots(int w, int h, int f) {
+    return insert_warps(w, h, f) == 24 ? 184 : 304;
 }
-SBF_SIZE_FN int insert_cta_bytes(int w, int h) { return kThreads / 32 * insert_warp_bytes(w, h); }
+SBF_SIZE_FN int insert_warp_bytes(int w, int h, int f) {
+    return insert_pool_slots(w, h, f) * (32 + 4) + 32 * 32;
+}
+SBF_SIZE_FN int insert_cta_bytes(int w, int h, int f) {
+    return kThreads / 32 * insert_warp_bytes(w, h, f);
+}
 
 // A record of a ragged launch: bytes [offset, offset + bytes) of the input.
 // Same layout as sbf_record_range of the C ABI.
@@ -129,8 +159,8 @@ struct KernelSet {
     const void* query_ragged;
     // Dynamic shared memory of the insert and query kernels: the tile
     // kernels' flush ring and shard pool; none for the generic kernels.
-    int smem_insert = insert_cta_bytes(k - m + 1, h);
-    int smem_query = query_cta_bytes(k - m + 1, h);
+    int smem_insert = insert_cta_bytes(k - m + 1, h, k - s + 1);
+    int smem_query = query_cta_bytes(k - m + 1, h, k - s + 1);
     bool jit = false;    // loaded from a run-time compiled library
     int jit_occupancy = 4;  // resident CTAs per SM assumed for run-time compiled sets
     const void* fn(int which) const {

@@ -813,7 +813,7 @@ __device__ __forceinline__ uint32_t query_strip(uint32_t code_mem, uint32_t stri
                                                 uint32_t vmask, uint32_t shard_mask,
                                                 const uint64_t* words, uint32_t run_mem) {
     constexpr int F = C::F;
-    constexpr uint32_t kPoolSlots = query_pool_slots(C::W, C::H);
+    constexpr uint32_t kPoolSlots = query_pool_slots(C::W, C::H, C::F);
     static_assert(kPoolSlots * 32 >= 32 * 128, "the run lists fit the pool");
     const uint32_t lane = threadIdx.x & 31;
     uint32_t result = 0;
@@ -1051,7 +1051,7 @@ __device__ __forceinline__ void insert_strip_runs(uint32_t code_mem, uint32_t st
                                                   uint64_t* words, uint32_t run_mem,
                                                   const uint64_t* onehot) {
     constexpr int F = C::F;
-    constexpr uint32_t kPoolSlots = insert_pool_slots(C::W, C::H);
+    constexpr uint32_t kPoolSlots = insert_pool_slots(C::W, C::H, C::F);
     static_assert(kPoolSlots * 32 >= 32 * 128, "the run lists fit the pool");
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t ids = run_mem + 32 * kPoolSlots;
@@ -1316,10 +1316,9 @@ __device__ __forceinline__ void tally_records(const TileParams& p, uint32_t firs
 // 488 us against 433, 10 M reads 5.95 ms against 5.12; with a CTA per tile of
 // 256 threads 452 and 5.38, of 64 threads 453 and 5.32).
 template <class C, bool kQuery, bool kDense, bool kRagged>
-__global__ void __launch_bounds__(kThreads, (kQuery ? query_24_warps(C::W, C::H)
-                                                    : insert_24_warps(C::W, C::H))
-                                                ? 24 * 32 / kThreads
-                                                : 16 * 32 / kThreads)
+__global__ void __launch_bounds__(kThreads, (kQuery ? query_warps(C::W, C::H, C::F)
+                                                    : insert_warps(C::W, C::H, C::F)) *
+                                                   32 / kThreads)
     tile_kernel(TileParams p) {
     constexpr int kCodeWords = C::kCodeWords;
     __shared__ alignas(128) uint8_t stage[C::kStageBytes];
@@ -1428,7 +1427,7 @@ __global__ void __launch_bounds__(kThreads, (kQuery ? query_24_warps(C::W, C::H)
             } else if (C::W == 1 && p.shard_mask < (32u << 20) / 32) {
                 hits = query_strip_direct<C>(code_mem, tid, vmask, p.shard_mask, p.words);
             } else {
-                constexpr int kWarpBytes = query_warp_bytes(C::W, C::H);
+                constexpr int kWarpBytes = query_warp_bytes(C::W, C::H, C::F);
                 hits = query_parts<C>(code_mem, vmask, p.shard_mask, p.words,
                                       smem_addr(slots) + (tid >> 5) * kWarpBytes);
             }
@@ -1437,7 +1436,7 @@ __global__ void __launch_bounds__(kThreads, (kQuery ? query_24_warps(C::W, C::H)
             if constexpr (kRagged) n_pos += __popc(hits & vmask);
             if (p.out_bits) store_strip_bits<C>(hits, p.out_bits, first_kmer, p.n_kmers);
         } else {
-            constexpr int kWarpBytes = insert_warp_bytes(C::W, C::H);
+            constexpr int kWarpBytes = insert_warp_bytes(C::W, C::H, C::F);
             insert_parts<C>(code_mem, vmask, p.shard_mask, p.words,
                             smem_addr(slots) + (tid >> 5) * kWarpBytes, onehot);
         }
