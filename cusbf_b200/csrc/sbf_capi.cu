@@ -423,7 +423,7 @@ extern "C" int sbf_filter_create(uint32_t k, uint32_t s, uint32_t m, uint32_t ha
         for (int i = 0; i < 6 && ks->jit; ++i) {
             const int dyn = ks->smem(i);
             int occ = 0;
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fns[i], kThreads, dyn) !=
+            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fns[i], ks->threads(i), dyn) !=
                     cudaSuccess ||
                 occ < 1) {
                 cudaGetLastError();
@@ -444,7 +444,7 @@ extern "C" int sbf_filter_create(uint32_t k, uint32_t s, uint32_t m, uint32_t ha
             }
             e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&f->occupancy[i],
                                                               reinterpret_cast<const void*>(fns[i]),
-                                                              kThreads, dyn);
+                                                              ks->threads(i), dyn);
             if (e != cudaSuccess) rc = cuda_fail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
             if (f->occupancy[i] < 1) f->occupancy[i] = 1;
         }

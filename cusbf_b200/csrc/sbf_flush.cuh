@@ -13,15 +13,18 @@ namespace sbf {
 // slot: one L2 sector operation instead of four 8-byte atomics.  Each thread
 // cycles through kFlushSlots slots; before reusing a slot it waits until the
 // bulk operation issued kFlushSlots flushes earlier has read it.
+// A CTA of `Threads`.
+template <int Threads>
 struct FlushRing {
-    uint64_t* slot0;  // this thread's slot 0; slot k at slot0 + k * kThreads * 4
+    uint64_t* slot0;  // this thread's slot 0; slot k at slot0 + k * Threads * 4
     uint32_t count;
 };
 
+template <int Threads>
 __device__ __forceinline__ void flush_run(uint64_t* words, uint32_t shard, const uint64_t a[4],
-                                          FlushRing& ring) {
+                                          FlushRing<Threads>& ring) {
     static_assert(kFlushSlots == 8, "wait_group.read immediate below assumes 8 slots");
-    uint64_t* slot = ring.slot0 + (ring.count & (kFlushSlots - 1)) * (kThreads * 4);
+    uint64_t* slot = ring.slot0 + (ring.count & (kFlushSlots - 1)) * (Threads * 4);
     asm volatile("cp.async.bulk.wait_group.read 7;" ::: "memory");
     *reinterpret_cast<ulonglong2*>(slot) = make_ulonglong2(a[0], a[1]);
     *reinterpret_cast<ulonglong2*>(slot + 2) = make_ulonglong2(a[2], a[3]);

@@ -112,11 +112,13 @@ __device__ __forceinline__ uint32_t eval_kmer(const GenericCfg& c, uint32_t shar
 // have none and use four 8-byte atomics.
 struct RuntimeGen {
     static constexpr bool kBulkFlush = false;
+    static constexpr int kRaggedInsertThreads = kThreads;
     __device__ __forceinline__ static GenericCfg get(const TileParams& p) { return p.gen; }
 };
 template <int K, int S, int M, int H, int Bits, int Width, int Alphabet>
 struct FixedGen {
     static constexpr bool kBulkFlush = true;
+    static constexpr int kRaggedInsertThreads = ragged_ring_threads(K - M + 1, Width);
     static constexpr int kK = K, kS = S, kM = M, kH = H, kBits = Bits;
     __device__ __forceinline__ static GenericCfg get(const TileParams&) {
         return GenericCfg{K, S, M, H, Bits, Width, Alphabet};
@@ -134,10 +136,11 @@ __device__ __forceinline__ void smer_value_masks(uint32_t h, uint64_t sm, uint64
 }
 
 template <class G, bool kQuery, bool kDense, bool kRagged>
-__global__ void __launch_bounds__(kThreads) generic_kernel(TileParams p) {
+__global__ void __launch_bounds__(kRagged && !kQuery ? G::kRaggedInsertThreads : kThreads)
+    generic_kernel(TileParams p) {
     const GenericCfg c = G::get(p);
     extern __shared__ __align__(16) uint64_t flush_slots[];
-    FlushRing ring{flush_slots + 4 * threadIdx.x, 0u};
+    FlushRing<kRagged && !kQuery ? G::kRaggedInsertThreads : kThreads> ring{flush_slots + 4 * threadIdx.x, 0u};
     (void)ring;
     const uint64_t n = p.n_kmers;
     const uint64_t n_strips = (n + kStrip - 1) / kStrip;

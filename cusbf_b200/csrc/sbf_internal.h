@@ -78,6 +78,14 @@ SBF_SIZE_FN int insert_cta_bytes(int w, int h, int f) {
     return kThreads / 32 * insert_warp_bytes(w, h, f);
 }
 
+// Threads per CTA of the ragged inserts with flush rings (sbf_generic.cuh), for
+// windows of `w` m-mers and symbols of `width` bytes.  In us with 256 / 128: 64 M
+// residues of <12,10,10,4> 898 / 1023, of <8,6,8,4> 1161 / 1278; 48 M triplets of
+// <10,8,5,4> 853 / 920, of <6,5,6,4> (one m-mer a window) 1339 / 1211.
+SBF_SIZE_FN int ragged_ring_threads(int w, int width) {
+    return width > 1 && w == 1 ? kThreads : 256;
+}
+
 // A record of a ragged launch: bytes [offset, offset + bytes) of the input.
 // Same layout as sbf_record_range of the C ABI.
 struct DevRange {
@@ -173,10 +181,12 @@ struct KernelSet {
     bool is_tile(int which) const {
         return !generic && !(generic_dense && (which == 2 || which == 3));
     }
+    int ragged_insert_threads = kThreads;  // of a generic set
+    int threads(int which) const { return which == 4 ? ragged_insert_threads : kThreads; }
     int smem(int which) const {
         const bool query = (which & 1) != 0;
         if (!generic && !is_tile(which)) return query ? 0 : kInsertSlotBytes;
-        return query ? smem_query : smem_insert;
+        return query ? smem_query : smem_insert / kThreads * threads(which);
     }
 };
 

@@ -347,6 +347,7 @@ const KernelSet* jit_kernels(int k, int s, int m, int h, int alphabet, int devic
             // ring's dynamic shared memory, queries none.
             e->ks.generic = true;
             e->ks.smem_insert = kInsertSlotBytes;
+            e->ks.ragged_insert_threads = ragged_ring_threads(k - m + 1, static_cast<int>(jc.width));
             e->ks.smem_query = 0;
             e->ks.jit_occupancy = 8;
         }

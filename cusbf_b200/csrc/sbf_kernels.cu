@@ -220,7 +220,7 @@ cudaError_t launch_set_kernel(const KernelSet* ks, const void* fn, unsigned grid
                               const TileParams& p, cudaStream_t stream) {
     TileParams copy = p;
     void* args[] = {&copy};
-    return cudaLaunchKernel(fn, dim3(grid), dim3(kThreads), args, ks->smem(which), stream);
+    return cudaLaunchKernel(fn, dim3(grid), dim3(ks->threads(which)), args, ks->smem(which), stream);
 }
 
 }  // namespace sbf

@@ -206,16 +206,20 @@ TileParams ragged_params(const sbf_filter* f, bool query, const uint8_t* d_seq,
 // the tile's records were exposed: contigs 1030 us against 925, reads 2020
 // against 1940, and 1007 / 2181 with a resident grid, whose tiles the CTAs
 // share unevenly).  The generic kernels load nothing ahead and take a CTA per
-// tile (64 M residues of <8,6,8,4>: insert 1285 us, with four tiles a CTA 1388,
-// with a resident grid 1485).  `ctas` limits the warps per SM (limited_ctas).
+// tile of their own size (64 M residues of <8,6,8,4>: insert 1161 us, with a
+// resident grid 1262); only triplets' inserts with CTAs of 256 threads keep a
+// resident grid (48 M triplets of <10,8,5,4>: 853 us, with a CTA per tile 874).
+// `ctas` limits the warps per SM (limited_ctas).
 static unsigned ragged_grid(const sbf_filter* f, bool query, uint64_t n_tiles, uint32_t ctas) {
     const int which = query ? kQueryRagged : kInsertRagged;
     const uint64_t resident =
         static_cast<uint64_t>(f->sms) *
-        limited_ctas(ctas, static_cast<uint32_t>(f->occupancy[which]), kThreads);
-    uint64_t grid = std::min<uint64_t>(n_tiles, resident);
-    const uint64_t tiles_each = f->ks->is_tile(which) ? 4 : 1;
-    if (ctas == 0)
+        limited_ctas(ctas, static_cast<uint32_t>(f->occupancy[which]),
+                     static_cast<uint32_t>(f->ks->threads(which)));
+    const uint64_t own = f->ks->threads(which) / kThreads;  // tiles of kTileKmers that a CTA covers
+    uint64_t grid = std::min<uint64_t>((n_tiles + own - 1) / own, resident);
+    const uint64_t tiles_each = f->ks->is_tile(which) ? 4 : own;
+    if (ctas == 0 && !(f->width > 1 && own > 1))
         grid = std::max<uint64_t>(
             grid, std::min<uint64_t>((n_tiles + tiles_each - 1) / tiles_each, 0x7FFFFFFFu));
     return static_cast<unsigned>(std::max<uint64_t>(grid, 1));

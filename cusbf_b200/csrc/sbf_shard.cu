@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(kThreads) apply_runs_kernel(const uint32_t* sh
                                                               uint64_t* words, uint64_t lo,
                                                               uint64_t hi, int* err) {
     extern __shared__ __align__(16) uint64_t ring_mem[];
-    FlushRing ring{ring_mem + 4 * threadIdx.x, 0u};
+    FlushRing<kThreads> ring{ring_mem + 4 * threadIdx.x, 0u};
     for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
          i += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
         const uint64_t sh = shards[i];
