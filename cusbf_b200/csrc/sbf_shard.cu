@@ -48,9 +48,8 @@ __device__ __forceinline__ void log_put(const RunLog& log, uint64_t at, uint32_t
 
 // Insert: the mask of window j is T_j = OR of the one-hot masks of its F
 // s-mers; a super-k-mer run (consecutive valid windows with equal shard)
-// accumulates acc = OR T_j and is handed to flush(end, shard, acc) with end
-// non-zero when the next window leaves the run.  With four s-mers per window,
-// flush is called on every window with `end` as its predicate.
+// accumulates acc = OR T_j and is handed to flush(shard, acc) once a window
+// leaves it.
 template <class C, class Flush>
 __device__ __forceinline__ void insert_strip(const uint32_t* c, uint32_t vmask,
                                              uint32_t shard_mask, const uint64_t* onehot,
@@ -76,7 +75,7 @@ __device__ __forceinline__ void insert_strip(const uint32_t* c, uint32_t vmask,
             smer_masks<C>(c, j + 3, m3, onehot);
             const bool valid = (vmask >> j) & 1u;
             const bool cont = valid && prev_valid && shard == prev_shard;
-            flush((prev_valid && !cont) ? 1u : 0u, prev_shard, acc);
+            if (prev_valid && !cont) flush(prev_shard, acc);
             const uint64_t keep = cont ? ~uint64_t{0} : uint64_t{0};
 #pragma unroll
             for (int w = 0; w < 4; ++w) {
@@ -97,7 +96,7 @@ __device__ __forceinline__ void insert_strip(const uint32_t* c, uint32_t vmask,
             smer_masks<C>(c, j + F - 1, mring[(j + F - 1) % F], onehot);
             const bool valid = (vmask >> j) & 1u;
             const bool cont = valid && prev_valid && shard == prev_shard;
-            if (prev_valid && !cont) flush(1u, prev_shard, acc);
+            if (prev_valid && !cont) flush(prev_shard, acc);
             const uint64_t keep = cont ? ~uint64_t{0} : uint64_t{0};
 #pragma unroll
             for (int w = 0; w < 4; ++w) {
@@ -110,78 +109,72 @@ __device__ __forceinline__ void insert_strip(const uint32_t* c, uint32_t vmask,
             prev_valid = valid;
         });
     }
-    if (prev_valid) flush(1u, prev_shard, acc);
+    if (prev_valid) flush(prev_shard, acc);
 }
 
-// The insert tile path with each super-k-mer run
-// appended to the CTA's shared-memory log; at the end of every tile the CTA
-// reserves a contiguous range of the global log with one atomic and copies
-// its records there.
+// The insert tile path with each super-k-mer run appended to the CTA's
+// shared-memory log; at the end the CTA reserves a contiguous range of the
+// global log with one atomic and copies its records there.  A CTA per tile, for
+// the reasons of tile_kernel: 64 Mbp 421 us, with a resident grid 528.
 template <class C>
 __global__ void __launch_bounds__(kThreads, 4) emit_kernel(TileParams p, RunLog log) {
     __shared__ alignas(16) uint8_t stage[kStageBytes];
     __shared__ uint32_t code[kCodeWords + 4];
     __shared__ uint32_t inval[kCodeWords + 4];
-    __shared__ unsigned int cta_n;
+    __shared__ unsigned int cta_n, cta_valid;
     __shared__ unsigned long long cta_base;
     __shared__ uint64_t onehot[64];
     extern __shared__ __align__(16) uint64_t dyn[];
     uint64_t* s_masks = dyn;                                          // [kLogRecords][4]
     uint32_t* s_shards = reinterpret_cast<uint32_t*>(dyn + 4 * kLogRecords);  // [kLogRecords]
     const int tid = threadIdx.x;
-    if (tid == 0) cta_n = 0;
-    onehot_init(onehot);  // published by the barrier at the top of the tile loop
-    unsigned long long n_valid = 0;
-    for (uint64_t tile = blockIdx.x; tile < p.n_tiles; tile += gridDim.x) {
-        TileGeom g = tile_geom<C, false>(p, tile);
-        g.hi = g.lo;  // no bulk copy: every readable byte by plain loads
-        __syncthreads();
-        fill_ragged<false>(p, g, stage);
-        __syncthreads();
-        for (int q = tid; q < kCodeWords; q += kThreads) {
-            uint32_t cw, iv;
-            encode_word<false>(g.off, stage, q, cw, iv);
-            code[q] = cw;
-            inval[q] = iv;
-        }
-        __syncthreads();
-        uint32_t c[kStripWords], iv[kStripWords];
-#pragma unroll
-        for (int q = 0; q < kStripWords; ++q) {
-            c[q] = code[tid * (kStrip / 16) + q];
-            iv[q] = inval[tid * (kStrip / 16) + q];
-        }
-        const int64_t first_kmer = g.s0 + static_cast<int64_t>(tid) * kStrip;
-        const uint64_t bits = static_cast<uint64_t>(iv[0]) | (static_cast<uint64_t>(iv[1]) << 16) |
-                              (static_cast<uint64_t>(iv[2]) << 32) |
-                              (static_cast<uint64_t>(iv[3]) << 48);
-        const uint32_t vmask = strip_valid<C>(bits, first_kmer, p.n_kmers);
-        n_valid += __popc(vmask);
-        if (vmask)
-            insert_strip<C>(c, vmask, p.shard_mask, onehot, [&](uint32_t end, uint32_t shard,
-                                                        const uint64_t* acc) {
-                if (!end) return;
-                const unsigned int i = atomicAdd(&cta_n, 1u);
-                if (i < static_cast<unsigned int>(kLogRecords)) {
-                    s_shards[i] = shard;
-                    *reinterpret_cast<ulonglong2*>(s_masks + 4 * i) = make_ulonglong2(acc[0], acc[1]);
-                    *reinterpret_cast<ulonglong2*>(s_masks + 4 * i + 2) =
-                        make_ulonglong2(acc[2], acc[3]);
-                } else {
-                    log_put(log, atomicAdd(log.count, 1ull), shard, acc);
-                }
-            });
-        __syncthreads();
-        const unsigned int n = min(cta_n, static_cast<unsigned int>(kLogRecords));
-        if (tid == 0) cta_base = n ? atomicAdd(log.count, static_cast<unsigned long long>(n)) : 0;
-        __syncthreads();
-        for (unsigned int i = tid; i < n; i += kThreads) log_put(log, cta_base + i, s_shards[i], s_masks + 4 * i);
-        __syncthreads();
-        if (tid == 0) cta_n = 0;
+    if (tid == 0) cta_n = cta_valid = 0;
+    onehot_init(onehot);
+    TileGeom g = tile_geom<C, false>(p, blockIdx.x);
+    g.hi = g.lo;  // no bulk copy: every readable byte by plain loads
+    fill_ragged<false>(p, g, stage);
+    __syncthreads();
+    for (int q = tid; q < kCodeWords; q += kThreads) {
+        uint32_t cw, iv;
+        encode_word<false>(g.off, stage, q, cw, iv);
+        code[q] = cw;
+        inval[q] = iv;
     }
+    __syncthreads();
+    uint32_t c[kStripWords], iv[kStripWords];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) n_valid += __shfl_down_sync(0xFFFFFFFFu, n_valid, o);
-    if ((tid & 31) == 0 && n_valid) atomicAdd(log.count + 1, n_valid);
+    for (int q = 0; q < kStripWords; ++q) {
+        c[q] = code[tid * (kStrip / 16) + q];
+        iv[q] = inval[tid * (kStrip / 16) + q];
+    }
+    const int64_t first_kmer = g.s0 + static_cast<int64_t>(tid) * kStrip;
+    const uint64_t bits = static_cast<uint64_t>(iv[0]) | (static_cast<uint64_t>(iv[1]) << 16) |
+                          (static_cast<uint64_t>(iv[2]) << 32) |
+                          (static_cast<uint64_t>(iv[3]) << 48);
+    const uint32_t vmask = strip_valid<C>(bits, first_kmer, p.n_kmers);
+    const uint32_t n_valid = __reduce_add_sync(0xFFFFFFFFu, static_cast<uint32_t>(__popc(vmask)));
+    if ((tid & 31) == 0) atomicAdd(&cta_valid, n_valid);
+    if (vmask)
+        insert_strip<C>(c, vmask, p.shard_mask, onehot, [&](uint32_t shard, const uint64_t* acc) {
+            const unsigned int i = atomicAdd(&cta_n, 1u);
+            if (i < static_cast<unsigned int>(kLogRecords)) {
+                s_shards[i] = shard;
+                *reinterpret_cast<ulonglong2*>(s_masks + 4 * i) = make_ulonglong2(acc[0], acc[1]);
+                *reinterpret_cast<ulonglong2*>(s_masks + 4 * i + 2) =
+                    make_ulonglong2(acc[2], acc[3]);
+            } else {
+                log_put(log, atomicAdd(log.count, 1ull), shard, acc);
+            }
+        });
+    __syncthreads();
+    const unsigned int n = min(cta_n, static_cast<unsigned int>(kLogRecords));
+    if (tid == 0) {
+        cta_base = n ? atomicAdd(log.count, static_cast<unsigned long long>(n)) : 0;
+        if (cta_valid) atomicAdd(log.count + 1, static_cast<unsigned long long>(cta_valid));
+    }
+    __syncthreads();
+    for (unsigned int i = tid; i < n; i += kThreads)
+        log_put(log, cta_base + i, s_shards[i], s_masks + 4 * i);
 }
 
 // ORs records whose shards lie in [lo, hi) into the filter, each with one
@@ -280,8 +273,7 @@ extern "C" int sbf_emit_runs_async(const sbf_filter_t* f, const char* d_seq, uin
     p.n_tiles = (n_kmers + kTileKmers - 1) / kTileKmers;
     p.err = f->d_err;
     RunLog log{d_shards, d_masks, capacity, reinterpret_cast<unsigned long long*>(d_count)};
-    const uint64_t grid = std::min<uint64_t>(p.n_tiles, static_cast<uint64_t>(f->sms) * 4);
-    es->fn<<<static_cast<unsigned>(grid), kThreads, kEmitSmem, st>>>(p, log);
+    es->fn<<<static_cast<unsigned>(p.n_tiles), kThreads, kEmitSmem, st>>>(p, log);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "emit_kernel");
     return SBF_OK;
 }
