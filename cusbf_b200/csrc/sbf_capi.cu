@@ -380,8 +380,8 @@ extern "C" int sbf_filter_create(uint32_t k, uint32_t s, uint32_t m, uint32_t ha
                          hashes);
     // Specialised tile kernels for the compiled DNA configurations; for any
     // other configuration, kernels compiled at run time (below, once the
-    // device is known: the tile kernels for DNA, the generic kernels with
-    // constant parameters for the other alphabets), or the
+    // device is known: the tile kernels for DNA and proteins, the generic
+    // kernels with constant parameters for the rest), or the
     // runtime-parameterised kernels when run-time compilation is not possible.
     const KernelSet* ks = alphabet == SBF_ALPHABET_DNA
                               ? find_kernels(static_cast<int>(k), static_cast<int>(s),

@@ -203,8 +203,4 @@ __device__ __forceinline__ void load_shard(const uint64_t* p, uint64_t& w0, uint
                  : "l"(p));
 }
 
-__device__ __forceinline__ void red_or(uint64_t* p, uint64_t v) {
-    asm volatile("red.relaxed.gpu.global.or.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-
 }  // namespace sbf

@@ -112,9 +112,10 @@ struct DevSizes {
     uint64_t n_ranges;
 };
 
-// One launch of a tile kernel.  Grid position g of tile n is
-// g = n * kTileKmers + (0 .. kTileKmers-1); it holds window (k-mer)
-// i = g + sym_base, and symbol i is the first base of that window.
+// One launch of a tile kernel.  With T windows a tile (StripKernel::tile_kmers:
+// kTileKmers, fewer with narrower strips), tile n has the grid positions
+// g = n * T + (0 .. T-1); position g holds window (k-mer) i = g + sym_base,
+// and symbol i is the first base of that window.
 struct TileParams {
     const uint8_t* input;    // device bytes (ASCII) or dense words viewed as bytes
     uint64_t input_bytes;    // readable bytes at `input`
@@ -152,11 +153,14 @@ enum : int {
     kDevErrRecordRange = 2,   // sharded insert: a run record outside the rank's shards
 };
 
-// Function table for one compiled configuration <K,S,M,H> (k = s = m = h = 0
-// for the generic table, whose kernels read TileParams::gen).
 #ifndef __CUDACC_RTC__
-// Kernels are launched with cudaLaunchKernel(fn, ...): a compiled kernel's
-// host stub, or a cudaKernel_t of a kernel compiled at run time (jit).
+// Which of a set's kernels: insert or query of bytes, dense words, records.
+enum { kInsertBytes, kQueryBytes, kInsertDense, kQueryDense, kInsertRagged, kQueryRagged };
+
+// Function table for one compiled configuration <K,S,M,H> (k = s = m = h = 0
+// for the generic table, whose kernels read TileParams::gen).  Kernels are
+// launched with cudaLaunchKernel(fn, ...): a compiled kernel's host stub, or a
+// cudaKernel_t of a kernel compiled at run time (jit).
 struct KernelSet {
     int k, s, m, h;
     const void* insert_bytes;
@@ -165,8 +169,9 @@ struct KernelSet {
     const void* query_dense;
     const void* insert_ragged;
     const void* query_ragged;
-    // Dynamic shared memory of the insert and query kernels: the tile
-    // kernels' flush ring and shard pool; none for the generic kernels.
+    // Dynamic shared memory of the insert and query kernels: the tile kernels'
+    // pools, the flush ring of the generic inserts compiled at run time, none
+    // for the other generic kernels.
     int smem_insert = insert_cta_bytes(k - m + 1, h, k - s + 1);
     int smem_query = query_cta_bytes(k - m + 1, h, k - s + 1);
     bool jit = false;    // loaded from a run-time compiled library
@@ -179,10 +184,12 @@ struct KernelSet {
     // Sets of generic kernels; protein tile sets have generic dense kernels.
     bool generic = false, generic_dense = false;
     bool is_tile(int which) const {
-        return !generic && !(generic_dense && (which == 2 || which == 3));
+        return !generic && !(generic_dense && (which == kInsertDense || which == kQueryDense));
     }
     int ragged_insert_threads = kThreads;  // of a generic set
-    int threads(int which) const { return which == 4 ? ragged_insert_threads : kThreads; }
+    int threads(int which) const {
+        return which == kInsertRagged ? ragged_insert_threads : kThreads;
+    }
     int smem(int which) const {
         const bool query = (which & 1) != 0;
         if (!generic && !is_tile(which)) return query ? 0 : kInsertSlotBytes;
@@ -197,9 +204,6 @@ inline uint64_t limited_ctas(uint32_t limit, uint32_t occupancy, uint32_t thread
     const uint64_t ctas = limit ? uint64_t{limit} * 256 / threads : occupancy;
     return ctas < 1 ? 1 : ctas < occupancy ? ctas : occupancy;
 }
-
-// Which of a set's kernels: insert or query of bytes, dense words, records.
-enum { kInsertBytes, kQueryBytes, kInsertDense, kQueryDense, kInsertRagged, kQueryRagged };
 
 // A kernel and the windows per thread it was compiled for.
 struct StripKernel {

@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(kThreads, 4) emit_kernel(TileParams p, RunLog 
 
 // ORs records whose shards lie in [lo, hi) into the filter, each with one
 // 32-byte bulk OR-reduction from the thread's shared-memory ring (one L2
-// operation per record, as the insert kernel flushes its runs); a record
+// operation per record); a record
 // outside the range sets the error word (it was routed to the wrong rank).
 __global__ void __launch_bounds__(kThreads) apply_runs_kernel(const uint32_t* shards,
                                                               const uint64_t* masks, uint64_t n,

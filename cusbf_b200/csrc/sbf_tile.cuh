@@ -25,7 +25,8 @@
 //   * Both list a strip's super-k-mer runs (consecutive windows that select
 //     one shard) and give the runs that hold a valid window consecutive slots
 //     of a per-warp shared-memory pool; a run that crosses into the next
-//     strip is one run.
+//     strip is one run.  (Windows of one or two m-mers go through the pool in
+//     parts of 8 windows.)
 //   * Query has the warp copy the runs' 32-byte shards to their slots with
 //     cp.async, a lane pair per shard (one request each), and tests the
 //     findere rule (all k-s+1 s-mers present) per window with byte permutes
